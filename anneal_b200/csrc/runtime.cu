@@ -643,6 +643,17 @@ int try_row_chain(anl_device* dev, const std::vector<Item>& items, size_t first,
     while (members.size() >= 2) {
         uint64_t k2 = fnv1a(&key, sizeof key, members.size());
         for (auto* m : members) { uint64_t h = structure_hash(*m); k2 = fnv1a(&h, sizeof h, k2); }
+        // A chain loads an operand that several members read once, for all of them: which operands coincide is part
+        // of what was compiled, and no structure hash holds it (every operand by the place its buffer comes first at).
+        {
+            std::map<uint32_t, uint32_t> first_at;
+            uint32_t place = 0;
+            for (auto* m : members)
+                for (size_t b = 1; b < m->bufs.size(); b++, place++) {
+                    const uint32_t at = first_at.insert({m->bufs[b].id, place}).first->second;
+                    k2 = fnv1a(&at, sizeof at, k2);
+                }
+        }
         auto f = dev->chains.find(k2);
         std::shared_ptr<ChainPlan> cp;
         if (f != dev->chains.end()) cp = f->second;

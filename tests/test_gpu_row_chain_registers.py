@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 from anneal_b200 import workloads as W
+from anneal_b200.tensor import Tensor
 from util import rel_err, schedule
 
 pytestmark = pytest.mark.gpu
@@ -67,3 +68,27 @@ def test_half_precision_cross_entropy(cuda, oracle, batch, classes):
         compare(cuda, oracle, m.graph(x, y).targets(), 2e-3, what=f"cross-entropy {batch}x{classes}")
     finally:
         R.MATERIALIZE_CONTRACTION_OPERANDS = False
+
+
+def _deviation(cuda, oracle, rows, cols, shared):
+    """sum((y - max(x))^2) a row, with y = x or another leaf of the same shape: item for item the same structure."""
+    x = Tensor.new_leaf((rows, cols)).set_data(W.normal(51, 1, rows * cols))
+    y = x if shared else Tensor.new_leaf((rows, cols)).set_data(W.normal(51, 2, rows * cols) + np.float32(3))
+    d = y.sub(x.max((1,)).reshape((rows, 1)).expand((rows, cols)))
+    items, ids, inputs = schedule([d.mul(d).sum((1,))])
+    before = cuda.stats()["kernels_launched"]
+    got = cuda.run(items, inputs)[ids[0]]
+    assert cuda.stats()["kernels_launched"] - before == 1
+    want = oracle.run(items, inputs)[ids[0]]
+    assert rel_err(got, want) <= tol(cols), (rows, cols, shared, rel_err(got, want))
+
+
+# a thread, a warp and a block a row, the next row fetched ahead, and rows that stay in memory
+@pytest.mark.parametrize("rows,cols", [(33, 12), (40, 300), (300, 1000), (1300, 2052), (130, 16400)])
+@pytest.mark.parametrize("first", [True, False])
+def test_chains_that_differ_only_in_what_they_share(cuda, oracle, rows, cols, first):
+    """A compiled chain is kept by its members' structure and by which of their operands coincide: on one device, either may
+    come first.  (Its own row count a direction, so that neither direction finds the other's kernels.)"""
+    rows += 0 if first else 1
+    _deviation(cuda, oracle, rows, cols, first)
+    _deviation(cuda, oracle, rows, cols, not first)
