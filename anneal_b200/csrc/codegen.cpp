@@ -683,6 +683,23 @@ struct Gen {
         }
         return cr == C && cs == 1;
     }
+    // Is parameter p read at element (row, sweep) of a dense matrix of C columns and nowhere else?
+    bool reads_own_row(int p, int64_t C) {
+        for (int i = 0; i < n; i++) {
+            if (N(i).op != OP_INDEX || i == dst || !is_live(i) || N(N(i).src[0]).op != OP_PARAM || N(N(i).src[0]).arg != p) continue;
+            const Lin f = flat_index(i);
+            bool row = false, sweep = false;
+            for (auto& t : f.t) {
+                const Atom& a = atoms[t.first];
+                if (a.kind != Atom::RANGE) return false;
+                if (a.node == loop_ranges[0] && t.second == C) row = true;
+                else if (a.node != loop_ranges[0] && t.second == 1 && !N(a.node).symbolic() && N(a.node).arg == C) sweep = true;
+                else return false;
+            }
+            if (f.c != 0 || f.t.size() != 2 || !row || !sweep) return false;
+        }
+        return true;
+    }
     // The sweeps of a chain stage all run over the same static extent C, one range each: C, and the row-contiguous loads
     // with the sweep variable they follow; 0 when the stage is not of this form, -1 when it sweeps nothing.
     int64_t row_extent(std::vector<int>& loads) {
@@ -2206,12 +2223,12 @@ bool render_row_chain(const std::vector<const Item*>& items, const std::vector<s
         body << code;
         if (piped && s == 0) body << "  @NEXT@\n";
         for (size_t b = 0; b < items[s]->bufs.size(); b++) {
-            bool is_chain_out = b == 0;      // written by this kernel: never const/restrict
-            std::string ty = std::string(is_chain_out ? "" : "const ") + buf_ctype(items[s]->bufs[b].dtype) + "*";
-            sig << (first_arg ? "" : ", ") << ty << " __restrict__ s" << s << "_data" << b << "_";
+            // written by this kernel: never const, and not restrict either, as two stages' results may share memory
+            std::string ty = b == 0 ? std::string(buf_ctype(items[s]->bufs[b].dtype)) + "*" : "const " + std::string(buf_ctype(items[s]->bufs[b].dtype)) + "* __restrict__";
+            sig << (first_arg ? "" : ", ") << ty << " s" << s << "_data" << b << "_";
             // device blocks are 256-byte aligned (pool granularity, 128-element view offsets)
             const std::string local = "s" + std::to_string(s) + "_data" + std::to_string(b);
-            aligned << "  " << ty << " __restrict__ " << local << " = (" << ty << ")__builtin_assume_aligned(" << local << "_, 16); (void)" << local << ";\n";
+            aligned << "  " << ty << " " << local << " = (" << ty << ")__builtin_assume_aligned(" << local << "_, 16); (void)" << local << ";\n";
             first_arg = false;
         }
     }
@@ -2243,6 +2260,14 @@ bool render_row_chain(const std::vector<const Item*>& items, const std::vector<s
         if (segments < 2) k << "  __syncthreads();\n";            // with two reductions, either's barrier keeps the other's segment
         k << "  }\n}\n";
     } else k << shift_decl("row") << loads.str() << stages << "}\n";
+    out.full_row = inner.back();
+    out.own_row.assign(items.size(), {});
+    for (size_t s = 0; s < items.size(); s++) {
+        Gen g(*items[s], opts);
+        if (!g.analyse()) { err = g.err; return false; }
+        for (size_t b = 0; b < items[s]->bufs.size(); b++)
+            out.own_row[s].push_back(out.full_row && b > 0 && rows > 0 && g.reads_own_row((int)b, items.back()->bufs[0].elems(0) / rows));
+    }
     out.blocks_per_sm = piped ? blocks : 0;
     out.smem_bytes = piped ? (unsigned)smem_at : 0u;
     out.source = k.str();
@@ -2253,6 +2278,32 @@ bool render_row_chain(const std::vector<const Item*>& items, const std::vector<s
     out.note = "row chain of " + std::to_string(items.size()) + " stages, " + std::to_string(rows) + " rows";
     if (held) out.note += ", " + std::to_string(row_bufs.size()) + " operands in registers, " + std::to_string(lanes) + " lanes a row";
     return true;
+}
+
+bool chain_overwrites(const std::vector<const Item*>& items, const std::vector<std::vector<std::pair<int, int>>>& chain_reads,
+                      const ChainRendered& r, const std::function<int(const BufDesc&, const BufDesc&)>& place) {
+    auto alike = [](const BufDesc& a, const BufDesc& b) { return a.dtype == b.dtype && a.elems(0) == b.elems(0); };
+    for (size_t w = 0; w < items.size(); w++) {
+        const BufDesc& o = items[w]->bufs[0];
+        const bool full = r.full_row && w + 1 == items.size();
+        // two results: a value a row each, one over the other, is written by the same thread in order
+        for (size_t v = 0; v < w; v++) {
+            const int at = place(o, items[v]->bufs[0]);
+            if (at && (at != 1 || full || !alike(o, items[v]->bufs[0]))) return true;
+        }
+        // A result over an operand: only a whole row over the very elements that the same row has been read from.  A value
+        // a row would need the operand read at the row's index, and by all threads before the first of them stores.
+        for (size_t m = 0; m < items.size(); m++)
+            for (size_t b = 1; b < items[m]->bufs.size(); b++) {
+                const BufDesc& in = items[m]->bufs[b];
+                bool from_register = false;
+                for (auto& pr : chain_reads[m]) from_register = from_register || pr.first == (int)b;
+                if (from_register || o.id == in.id) continue;
+                const int at = place(o, in);
+                if (at && !(at == 1 && full && alike(o, in) && r.own_row[m][b])) return true;
+            }
+    }
+    return false;
 }
 
 bool render_cuda(const Item& item, const CodegenOpts& opts, Rendered& out, std::string& err) {

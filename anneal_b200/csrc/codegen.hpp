@@ -2,6 +2,7 @@
 // reference's Lower + RenderWGSL pair (codegen/lower.go:98-105, codegen/wgsl.go:36-39).
 #pragma once
 #include <cstdint>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -114,12 +115,19 @@ struct ChainRendered {
     int blocks_per_sm = 0;         // > 0: that many blocks an SM walk the rows (at most one block a row)
     unsigned smem_bytes = 0;
     bool held = false;             // the row's operands sit in registers: each is read from memory once
+    bool full_row = false;         // the last stage writes a whole row
+    std::vector<std::vector<char>> own_row;   // [stage][parameter]: read at element (row, sweep) of the last stage's dense matrix only
 };
 // True when `items` (in schedule order, at least two) form such a chain.  `ext_reads[k]` must list,
 // for stage k, which of its input parameters are outputs of EARLIER stages of the chain, as
 // (parameter number, producing stage).  Kernel arguments: every stage's buffers in order.
 bool render_row_chain(const std::vector<const Item*>& items, const std::vector<std::vector<std::pair<int, int>>>& chain_reads,
                       const CodegenOpts& opts, ChainRendered& out, std::string& err);
+// Buffers may share memory (`place` says how two of them lie: 0 apart, 1 at the same address, 2 otherwise overlapping),
+// which is sound while the members run one after the other.  In one launch the blocks are at different members: true when
+// one of them could write over what another still reads, or over another's result.
+bool chain_overwrites(const std::vector<const Item*>& items, const std::vector<std::vector<std::pair<int, int>>>& chain_reads,
+                      const ChainRendered& r, const std::function<int(const BufDesc&, const BufDesc&)>& place);
 
 // Hash of everything that determines the rendered source (node table, buffer dtypes and
 // shapes) and nothing that does not (buffer ids, slots).

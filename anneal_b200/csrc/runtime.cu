@@ -675,15 +675,13 @@ int try_row_chain(anl_device* dev, const std::vector<Item>& items, size_t first,
             }
             dev->chains[k2] = cp;
         }
-        // slots share memory: a block may finish its row only into memory that no other row of the chain still reads
-        bool clash = false;
-        for (auto* w : members)
-            for (size_t m = 0; m < members.size() && cp; m++)
-                for (size_t b = 1; b < members[m]->bufs.size(); b++) {
-                    const BufDesc &o = w->bufs[0], &in = members[m]->bufs[b];
-                    if (o.id != in.id && t.bufs[o.id].ptr == t.bufs[in.id].ptr && (o.elems(0) != in.elems(0) || o.dtype != in.dtype)) clash = true;
-                }
-        if (cp && !clash) {
+        // slots share memory, and a caller may place an output over an input
+        auto place = [&](const BufDesc& a, const BufDesc& b) {
+            const DevBuf &p = t.bufs[a.id], &q = t.bufs[b.id];
+            const char *pa = (const char*)p.ptr, *pb = (const char*)q.ptr;
+            return pa == pb ? 1 : pa < pb + q.bytes && pb < pa + p.bytes ? 2 : 0;
+        };
+        if (cp && !chain_overwrites(members, reads, cp->r, place)) {
             std::vector<void*> ptrs;
             for (auto* m : members) for (auto& b : m->bufs) ptrs.push_back(t.bufs[b.id].ptr);
             std::vector<void*> args;
@@ -1268,7 +1266,13 @@ static int lower_chain_impl(const uint8_t* blob, size_t blob_len, int first, int
         reads.push_back(rd);
     }
     ChainRendered r; CodegenOpts o;
-    if (!render_row_chain(members, reads, o, r, err)) { if (note && note_cap) std::snprintf(note, note_cap, "%s", err.c_str()); return ANL_ERR_UNSUPPORTED; }
+    if (render_row_chain(members, reads, o, r, err)) {
+        std::map<uint32_t, int> slots;
+        for (auto& it : items) if (it.bufs[0].slot >= 0) slots[it.bufs[0].id] = it.bufs[0].slot;
+        auto place = [&](const BufDesc& a, const BufDesc& b) { auto p = slots.find(a.id), q = slots.find(b.id); return p != slots.end() && q != slots.end() && p->second == q->second ? 1 : 0; };
+        if (chain_overwrites(members, reads, r, place)) err = "chain: a stage writes memory that another row may still read";
+    }
+    if (!err.empty()) { if (note && note_cap) std::snprintf(note, note_cap, "%s", err.c_str()); return ANL_ERR_UNSUPPORTED; }
     if (src && src_cap) { size_t n = std::min(src_cap - 1, r.source.size()); std::memcpy(src, r.source.data(), n); src[n] = 0; }
     if (src_len) *src_len = r.source.size();
     if (note && note_cap) std::snprintf(note, note_cap, "%s", r.note.c_str());
