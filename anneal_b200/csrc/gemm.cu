@@ -40,7 +40,6 @@ static const char* const kSmallKernelSource =
 constexpr int BM = 128, BK = 64;
 constexpr int A_TILE_BYTES = BM * BK * 2;          // 16 KiB
 constexpr int PAIR_THREADS = 320;        // two-CTA kernel: producer, MMA issuer and eight epilogue warps
-constexpr int SMALL_THREADS = 256;
 
 struct GemmPlan {
     Contraction c;
@@ -288,7 +287,7 @@ PairVariant choose_variant(anl_device* dev, const GemmPlan& gp_in, int64_t M) {
 // ── the run-time compiled one-CTA kernel ──────────────────────────────────────────────────────
 namespace {
 
-struct SmallVariant { bool a_mn, b_mn; int nt, prows, stages, splits; bool tf32; };
+struct SmallVariant { bool a_mn, b_mn; int nt, prows, stages, splits, chunk; bool tf32; int threads() const { return chunk ? 320 : 256; } };
 // k extent the 3 x TF32 form accumulates in tensor memory before adding to the output in f32.  Measured on
 // 4096 x 2048 x 8192 (error against float64, of the largest output): 1024 -> 7.6e-6 at 226 TFLOP/s,
 // 512 -> 3.5e-6 at 207, 256 -> 1.7e-6 at 146; the reference's serial f32 loop: 3.6e-6 (9.4e-6 at K = 65536).
@@ -302,7 +301,6 @@ int small_smem_bytes(const SmallVariant& v) {
     return std::max(ring, v.prows * (v.nt + 4) * 4) + 1024;
 }
 
-// nt = 0 when no slicing of K keeps every slice within what the 3 x TF32 form may accumulate at once
 SmallVariant choose_small(int64_t M, int64_t N, int64_t K, bool a_mn, bool b_mn, bool tf32) {
     SmallVariant v{};
     v.a_mn = a_mn; v.b_mn = b_mn; v.tf32 = tf32;
@@ -311,13 +309,13 @@ SmallVariant choose_small(int64_t M, int64_t N, int64_t K, bool a_mn, bool b_mn,
     if (!a_mn && M <= 64) v.prows = M <= 32 ? 32 : 64;
     const int parts = tf32 ? 2 : 1, bk = tf32 ? 32 : BK;
     const int64_t kblocks = (K + bk - 1) / bk, tm = (M + BM - 1) / BM;
+    const int most = tf32 ? 8 : 16;           // k-blocks of a chunk: 256 f32 or 1024 f16 terms
     double best = 1e30, best_ctas = 0;
     for (int nt : {128, 64, 32}) {
         if (b_mn && nt < 64) continue;
         for (int splits : {1, 2, 4, 8}) {
             if (splits > 1 && kblocks / splits < 2) break;
             const int64_t per = (kblocks + splits - 1) / splits;
-            if (tf32 && per * bk > kTf32ChunkK) continue;
             const double ctas = (double)(tm * ((N + nt - 1) / nt) * splits);
             // Time of the busiest SM in us, fitted to a sweep over 24 shapes from 1 x 4096 x 4096 to 2048-cubed: 3 for
             // the launch, prologue and epilogue; its k-blocks' loads at 100 bytes a ns for one CTA, 135 for two
@@ -330,7 +328,7 @@ SmallVariant choose_small(int64_t M, int64_t N, int64_t K, bool a_mn, bool b_mn,
             const double load = std::max(n * per * (double)(parts * (v.prows + nt) * 128) / (n > 1 && !alone ? 135e3 : 100e3), std::ceil(alone ? n : n / 2) * per * 0.25);
             double t = 3.0 + load + (splits == 1 ? 0.0 : splits == 2 ? 2.0 : splits == 4 ? 2.5 : 7.0);
             if (splits > 1 && ctas > 2 * 148) t *= 2;
-            if (t < best) { best = t; best_ctas = ctas; v.nt = nt; v.splits = splits; }
+            if (t < best) { best = t; best_ctas = ctas; v.nt = nt; v.splits = splits; v.chunk = per > most ? most : 0; }
         }
     }
     // two CTAs an SM, at most 110 KB each, unless each has an SM for itself or two stages do not fit that way
@@ -349,7 +347,7 @@ std::string small_source(const SmallVariant& v, const std::string& epilogue) {
     s += "#define CFG_NT " + std::to_string(v.nt) + "\n#define CFG_PROWS " + std::to_string(v.prows) + "\n";
     s += "#define CFG_STAGES " + std::to_string(v.stages) + "\n#define CFG_SPLITS " + std::to_string(v.splits) + "\n";
     s += "#define CFG_EPI " + std::string(epilogue.empty() ? "0" : "1") + "\n";
-    s += "#define CFG_TF32 " + std::string(v.tf32 ? "1" : "0") + "\n";
+    s += "#define CFG_TF32 " + std::string(v.tf32 ? "1" : "0") + "\n#define CFG_CHUNK " + std::to_string(v.chunk) + "\n";
     s += epilogue;
     s += kSmallKernelSource;
     return s;
@@ -357,7 +355,7 @@ std::string small_source(const SmallVariant& v, const std::string& epilogue) {
 
 int get_small_kernel(anl_device* dev, const SmallVariant& v, const std::string& epilogue, CUfunction* fn) {
     char head[96];
-    std::snprintf(head, sizeof head, "s%d,%d,%d,%d,%d,%d,%d|", v.nt, v.prows, v.stages, v.splits, (int)v.a_mn, (int)v.b_mn, (int)v.tf32);
+    std::snprintf(head, sizeof head, "s%d,%d,%d,%d,%d,%d,%d,%d|", v.nt, v.prows, v.stages, v.splits, v.chunk, (int)v.a_mn, (int)v.b_mn, (int)v.tf32);
     const std::string key = head + epilogue;
     auto hit = dev->pair_kernels.find(key);
     if (hit != dev->pair_kernels.end()) { *fn = (CUfunction)hit->second; return ANL_OK; }
@@ -517,14 +515,15 @@ int gemm_tf32_source(const Plan& plan, std::string& out, std::string& note) {
     return ANL_OK;
 }
 
-// The one-CTA kernel for f32 contractions with few tiles, where the slices of K it may accumulate cover K.  Measured against
-// the pair kernel (and the launch that adds its copies up), us with the operand splits: 256 x 4096 x 1024 29.7 / 36.8,
-// 64 x 4096 x 1024 25.6 / 31.7, 100 x 1000 x 700 17.4 / 29.7, 600-cubed 19.5 / 30.7, 512 x 4096 x 1024 37.9 / 46.0,
-// 2048 x 1024 x 1024 35.7 / 45.9 (32 tiles), 256 x 1024 x 4096 38.0 / 38.9; the other way 1024 x 4096 x 1024 60.4 / 58.4
-// (64 tiles) and 1024 x 1024 x 8192 198 / 126 (K in eight slices).
+// The one-CTA kernel for f32 contractions with few tiles.  Measured against the pair kernel (and the launch that adds its
+// copies up), us with the operand splits and the events: 256 x 4096 x 1024 31.7 / 35.8, 64 x 4096 x 1024 25.6 / 31.7,
+// 100 x 1000 x 700 17.4 / 29.7, 600-cubed 19.5 / 29.7, 1024-cubed 29.7 / 34.8, 512 x 4096 x 1024 39.9 / 46.1, 2048 x 1024 x 1024
+// 39.9 / 46.1 (32 tiles), 1024 x 1024 x 2048 44.0 / 46.0, 300 x 1024 x 4096 44.1 / 44.0; the other way 256 x 1024 x 4096 42.0 / 37.9
+// and 40 x 1024 x 4096 37.9 / 31.7 (the pair kernel has 16 slices where a cluster has 4), 1024 x 4096 x 1024 (64 tiles) and
+// 1024 x 1024 x 8192 198 / 126.  Its error is no larger there: chunks of 256 terms, where the pair kernel takes 256 to 1024.
 static bool tf32_small_takes(int64_t M, int64_t N, int64_t K) {
     const int64_t tiles = ((M + 255) / 256) * ((N + 255) / 256);
-    return tiles <= 36 && K <= 4096 && choose_small(M, N, K, false, false, true).nt > 0;
+    return tiles <= 36 && K <= 4096;
 }
 
 static int launch_gemm_tf32x3(anl_device* dev, const GemmPlan& gp, const float* a, const float* b, float* d, int64_t M, int64_t K,
@@ -575,7 +574,7 @@ static int launch_gemm_tf32x3(anl_device* dev, const GemmPlan& gp, const float* 
         g.status = dev->gemm_status_dev;
         const int64_t ctas = (int64_t)g.tiles_m * ((N + v.nt - 1) / v.nt) * v.splits;
         void* params[5] = {&ma_hi, &mb_hi, &ma_lo, &mb_lo, &g};
-        if ((rc = launch_kernel(dev, fn, KernelShape{(unsigned)ctas, 1, 1, SMALL_THREADS, 1, 1, (unsigned)small_smem_bytes(v), (unsigned)v.splits}, stream, params, true, "gemm_f16_tcgen05_small (f32)"))) return done(rc);
+        if ((rc = launch_kernel(dev, fn, KernelShape{(unsigned)ctas, 1, 1, (unsigned)v.threads(), 1, 1, (unsigned)small_smem_bytes(v), (unsigned)v.splits}, stream, params, true, "gemm_f16_tcgen05_small (f32)"))) return done(rc);
         dev->stats.gemm_launched++;
         return done(ANL_OK);
     }
@@ -699,7 +698,7 @@ int launch_gemm(anl_device* dev, const Plan& plan, void* const* bufs, int64_t sy
         if (ctas > 0x7fffffffLL) return done(dev->fail(ANL_ERR_LIMIT, "gemm: grid too large"));
         g.b_settled = b_settled && !gp.pad_b;
         void* params[3] = {&ma, &mb, &g};
-        if ((rc = launch_kernel(dev, fn, KernelShape{(unsigned)ctas, 1, 1, SMALL_THREADS, 1, 1, (unsigned)small_smem_bytes(v), (unsigned)v.splits}, stream, params, true, "gemm_f16_tcgen05_small"))) return done(rc);
+        if ((rc = launch_kernel(dev, fn, KernelShape{(unsigned)ctas, 1, 1, (unsigned)v.threads(), 1, 1, (unsigned)small_smem_bytes(v), (unsigned)v.splits}, stream, params, true, "gemm_f16_tcgen05_small"))) return done(rc);
         dev->stats.gemm_launched++;
         return done(ANL_OK);
     }

@@ -19,10 +19,16 @@
 //
 // f32 operands (CFG_TF32 = 1) take the same kernel in the 3 x TF32 form of the pair kernel: every operand arrives as two
 // k-contiguous f32 arrays, hi and lo, a k-block is 32 deep and is staged as four parts, and three products are
-// accumulated on them.  No slice of K is longer than the 1024 that the pair kernel accumulates in tensor memory at
-// a time, and the slices are added in f32 round-to-nearest like its chunks, without copies of the output in memory
-// or a launch to add them up: 256 x 4096 x 1024 36.8 -> 29.7 us
-// alone, with the operand splits and the events.
+// accumulated on them, without copies of the output in memory or a launch to add them up.
+//
+// Tensor memory cuts each partial sum instead of rounding it, an error that grows with the number of additions.  A
+// slice of more than CFG_CHUNK k-blocks is therefore accumulated in chunks of that many, in two accumulators by turns: eight
+// more warps than the two that load and multiply take each finished chunk to registers and add it to the ones before, in f32
+// round-to-nearest, while the next one is multiplied.  Error against float64 (rms with normal values | mean with positive
+// ones), slices of 1024 f32 terms in one go, in chunks of 256, on the pair kernel: 256 x 1024 x 4096 7.1e-6 | 1.1e-5, 1.7e-6 |
+// 2.3e-6, 1.7e-6 | 2.3e-6 (37.9, 42.0, 37.9 us alone, with the operand splits and the events); 2048 x 1024 x 1024 7.1e-6 | 1.1e-5,
+// 1.7e-6 | 2.3e-6, 3.5e-6 | 5.1e-6 (35.8, 39.9, 46.1 us).  Eight f16 slices of 8192 terms lost 4.7e-5 of a positive sum, in chunks
+// of 1024 they lose 5.6e-6, beside the 1.4e-4 rms of the rounding to f16 (40 x 4096 x 16384 34.8 and 38.9 us).
 //
 // With fewer than 128 rows only CFG_PROWS of them are loaded and staged; the MMA still reads 128 rows of
 // shared memory and the accumulator rows past the matrix are never stored (rows do not mix).
@@ -36,6 +42,7 @@
 //   CFG_PROWS            rows of A staged per k-block: 16, 32, 64 or 128 (128 when CFG_A_MN)
 //   CFG_STAGES           depth of the shared-memory ring of k-blocks
 //   CFG_SPLITS           CTAs per tile: 1, 2, 4 or 8
+//   CFG_CHUNK            k-blocks accumulated in tensor memory at a time; 0 when no slice is longer than a chunk
 //   CFG_TF32             1: f32 operands as hi and lo parts, f32 output (k-contiguous only, no fused consumer, no column sums)
 //   CFG_EPI              1 when a fused elementwise consumer has been prepended (gemm_pair_kernel.cuh says how)
 #pragma once
@@ -58,11 +65,11 @@ struct SmallGemmArgs {
 struct alignas(64) TensorMap { unsigned long long opaque[16]; };
 
 // a k-block is one 128-byte swizzle row of k: 64 f16 or 32 f32 elements; in the f32 form each operand is staged as hi, then lo
-constexpr int BM = 128, BK = CFG_TF32 ? 32 : 64, PARTS = CFG_TF32 ? 2 : 1, NT = CFG_NT, NSTAGE = CFG_STAGES, SPLITS = CFG_SPLITS, THREADS = 256;
+constexpr int BM = 128, BK = CFG_TF32 ? 32 : 64, PARTS = CFG_TF32 ? 2 : 1, NT = CFG_NT, NSTAGE = CFG_STAGES, SPLITS = CFG_SPLITS, CHUNK = CFG_CHUNK, THREADS = CHUNK ? 320 : 256;
 constexpr int P_PART = CFG_PROWS * 128, Q_PART = NT * 128, P_BYTES = PARTS * P_PART, STAGE_BYTES = P_BYTES + PARTS * Q_PART;
 static_assert(!(CFG_TF32 && (CFG_A_MN || CFG_B_MN || CFG_EPI)), "the f32 form takes k-contiguous operands and no consumer");
 constexpr int LDT = NT + 4;              // floats per row of the staged f32 tile: rows 16 bytes apart in the banks
-constexpr int TMEM_COLS = NT < 32 ? 32 : NT;
+constexpr int TMEM_COLS = CHUNK ? 2 * NT : NT;
 constexpr unsigned WAIT_LIMIT = 1u << 20;
 static_assert(!CFG_A_MN || CFG_PROWS == 128, "an m-contiguous operand is staged whole");
 static_assert(!CFG_B_MN || NT % 64 == 0, "an n-contiguous operand is staged in boxes of 64");
@@ -72,6 +79,7 @@ __device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) { asm vo
 __device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(unsigned bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 // Bounded wait: false when the phase did not complete within WAIT_LIMIT polls, or when another role of this
 // CTA has already given up.
 __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, const volatile int* failed) {
@@ -139,7 +147,7 @@ gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_con
 gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_constant__ TensorMap map_b, const SmallGemmArgs g) {
 #endif
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) unsigned long long full_bar[NSTAGE], empty_bar[NSTAGE], acc_full;
+    __shared__ __align__(8) unsigned long long full_bar[NSTAGE], empty_bar[NSTAGE], acc_full[2], acc_empty[2];
     __shared__ unsigned tmem_base_slot;
     __shared__ volatile int failed;
 
@@ -155,7 +163,7 @@ gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_con
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < NSTAGE; s++) { mbar_init(smem_u32(&full_bar[s]), 1); mbar_init(smem_u32(&empty_bar[s]), 1); }
-        mbar_init(smem_u32(&acc_full), 1);
+        for (int a = 0; a < 2; a++) { mbar_init(smem_u32(&acc_full[a]), 1); mbar_init(smem_u32(&acc_empty[a]), 8); }
         failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -222,15 +230,18 @@ gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_con
             bool ok = true;
             for (int it = 0; it < nkb; it++) {
                 if (!mbar_wait(smem_u32(&full_bar[stage]), phase, &failed)) { ok = false; *(volatile int*)g.status = 22; break; }
+                // chunk ch has accumulator ch & 1, which the chunk two before it has to have left
+                const int ch = CHUNK ? it / (CHUNK ? CHUNK : 1) : 0, kc = it - ch * CHUNK;
+                if (CHUNK && kc == 0 && !mbar_wait(smem_u32(&acc_empty[ch & 1]), ((unsigned)(ch >> 1) & 1u) ^ 1u, &failed)) { ok = false; *(volatile int*)g.status = 24; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const unsigned sp = smem_base + stage * STAGE_BYTES, sq = sp + P_BYTES;
+                const unsigned sp = smem_base + stage * STAGE_BYTES, sq = sp + P_BYTES, acc = tmem_base + (ch & 1) * NT;
 #if CFG_TF32
                 // A_lo · B_hi, A_hi · B_lo, A_hi · B_hi
 #pragma unroll
                 for (int pass = 0; pass < 3; pass++) {
                     const unsigned pp = pass == 0 ? sp + P_PART : sp, pq = pass == 1 ? sq + Q_PART : sq;
 #pragma unroll
-                    for (int k = 0; k < 4; k++) umma_f16(tmem_base, make_desc(pp + k * 32, 16, 1024), make_desc(pq + k * 32, 16, 1024), idesc, (it | pass | k) != 0);
+                    for (int k = 0; k < 4; k++) umma_f16(acc, make_desc(pp + k * 32, 16, 1024), make_desc(pq + k * 32, 16, 1024), idesc, (kc | pass | k) != 0);
                 }
 #else
 #pragma unroll
@@ -239,22 +250,59 @@ gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_con
                     // 128 bytes, 64-wide m/n groups one box apart.
                     const unsigned long long ad = CFG_A_MN ? make_desc(sp + k * 2048, BK * 128, 1024) : make_desc(sp + k * 32, 16, 1024);
                     const unsigned long long bd = CFG_B_MN ? make_desc(sq + k * 2048, BK * 128, 1024) : make_desc(sq + k * 32, 16, 1024);
-                    umma_f16(tmem_base, ad, bd, idesc, (it | k) != 0);
+                    umma_f16(acc, ad, bd, idesc, (kc | k) != 0);
                 }
 #endif
                 umma_commit(smem_u32(&empty_bar[stage]));
+                if (it + 1 == nkb || (CHUNK && kc + 1 == CHUNK)) umma_commit(smem_u32(&acc_full[ch & 1]));
                 if (++stage == NSTAGE) { stage = 0; phase ^= 1; }
             }
-            if (ok) umma_commit(smem_u32(&acc_full));
-            else failed = 1;
+            if (!ok) failed = 1;
         }
     }
     __syncwarp();
 
+#if CFG_CHUNK
+    // ── the eight other warps: a quadrant of the accumulators each, half of the columns, from chunk to chunk in registers and
+    // then to shared memory.  When the last chunk is complete, every TMA write has been consumed and every MMA has read
+    // its operands: the ring's memory is free. ──
+    if (warp >= 2) {
+        const int quad = warp & 3, half = (warp - 2) >> 2;
+        const bool used = m0 + quad * 32 < g.M;
+        const int chunks = (nkb + CHUNK - 1) / CHUNK;
+        float sum[NT / 2];
+        bool ok = true;
+        for (int ch = 0; ch < chunks && ok; ch++) {
+            ok = mbar_wait(smem_u32(&acc_full[ch & 1]), (unsigned)(ch >> 1) & 1u, &failed);
+            if (!ok && lane == 0) { *(volatile int*)g.status = 23; failed = 1; }
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (used) {
+#pragma unroll
+                for (int c = 0; c < NT / 32; c++) {
+                    unsigned v[16];
+                    tmem_ld16(tmem_base + ((unsigned)(quad * 32) << 16) + (ch & 1) * NT + half * (NT / 2) + c * 16, v);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int j = 0; j < 16; j++) sum[c * 16 + j] = ch ? sum[c * 16 + j] + __uint_as_float(v[j]) : __uint_as_float(v[j]);
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&acc_empty[ch & 1]));
+        }
+        if (ok && used) {
+            float4* const dst = reinterpret_cast<float4*>(tile + (quad * 32 + lane) * LDT + half * (NT / 2));
+#pragma unroll
+            for (int q = 0; q < NT / 8; q++) dst[q] = make_float4(sum[4 * q], sum[4 * q + 1], sum[4 * q + 2], sum[4 * q + 3]);
+        }
+    }
+#else
     // ── every warp: its quadrant of the accumulator, half of the columns, to shared memory ──
     // The accumulator is complete, so every TMA write has been consumed and every MMA has read its operands: the
     // ring's memory is free.
-    bool ok = mbar_wait(smem_u32(&acc_full), 0, &failed);
+    bool ok = mbar_wait(smem_u32(&acc_full[0]), 0, &failed);
     if (!ok && lane == 0) { *(volatile int*)g.status = 23; failed = 1; }
     ok = __all_sync(0xffffffffu, ok);
     const int quad = warp & 3, half = warp >> 2;
@@ -272,6 +320,7 @@ gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_con
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     }
+#endif
     __syncthreads();
     if (SPLITS > 1) cluster_sync_all();                  // all partial tiles are in place
 

@@ -78,3 +78,42 @@ def test_f32_form(cuda, M, N, K, layout):
     ref = am @ bm.T
     assert np.abs(y - ref).max() <= 1e-5 * np.abs(ref).max()
     assert np.array_equal(cuda.run(items, inputs)[ids[0]].reshape(M, N), y)
+
+
+def _bias(cuda, M, N, K, dtype, layout="KK"):
+    """Mean relative error against float64 of sums of K positive terms, and the standard error of that mean."""
+    gen = np.random.default_rng(K)
+    scale = np.sqrt(2000 / (2.25 * K)) if dtype is dtypes.float16 else 1.0        # f16 outputs near 2000
+    np_type = np.float16 if dtype is dtypes.float16 else np.float32
+    am, bm = ((gen.uniform(1, 2, (rows, K)) * scale).astype(np_type).astype(np.float32) for rows in (M, N))
+    f = lambda m, kc: (Tensor.new_leaf(m.shape, dtype).set_data(m.reshape(-1)) if kc else Tensor.new_leaf(m.shape[::-1], dtype).set_data(m.T.reshape(-1)).permute((1, 0)))
+    items, ids, inputs = schedule([f(am, layout[0] == "K").matmul(f(bm, layout[1] == "K").permute((1, 0)))])
+    before = cuda.stats()["gemm_launched"]
+    y = cuda.run(items, inputs)[ids[0]].reshape(M, N)
+    assert cuda.stats()["gemm_launched"] == before + 1
+    assert np.array_equal(cuda.run(items, inputs)[ids[0]].reshape(M, N), y)
+    ref = am.astype(np.float64) @ bm.astype(np.float64).T
+    e = y / ref - 1.0
+    return abs(e.mean()), e.std() / np.sqrt(e.size)
+
+
+# one tile of few columns; a chunk and a k-block, two chunks, slices of unequal length (one of them no longer than a
+# chunk); narrow, wide and partly empty tiles; the longest K of the route
+@pytest.mark.parametrize("M,N,K", [(256, 1024, 288), (256, 1024, 512), (64, 1024, 4096), (300, 1024, 4096), (2048, 1024, 1024), (512, 4096, 1024),
+                                   (256, 4096, 1000), (64, 1001, 4001), (1000, 300, 545)])
+def test_long_f32_sums_lose_no_more_than_one_chunk(cuda, M, N, K):
+    """The tensor cores cut each partial sum, so the mean error of a sum of positive terms grows with the additions that one
+    accumulator takes: K terms must show no more than the 256 of a chunk do (with a tenth and four standard errors in hand),
+    plus one rounding for each chunk added in f32."""
+    one, s1 = _bias(cuda, 256, 1024, 256, dtypes.float32)
+    many, s2 = _bias(cuda, M, N, K, dtypes.float32)
+    assert many <= 1.1 * one + 4 * (s1 + s2) + (K // 256) * 2.0 ** -25, (many, one)
+
+
+@pytest.mark.parametrize("M,N,K,layout", [(40, 1024, 65536, "KK"), (40, 1024, 9000, "MM"), (300, 40, 20001, "KK"), (1, 4096, 32768, "KK"), (77, 333, 8191, "MK"),
+                                          (256, 256, 16384, "KM"), (130, 96, 1100, "KK")])
+def test_long_f16_sums_lose_no_more_than_one_chunk(cuda, M, N, K, layout):
+    """The same with chunks of 1024 terms, 64 additions: each cuts less than 2^-22 of what has been added up so far, half of the
+    total on average, so 32 x 2^-22 in all, below the 2^-12 of the one rounding to f16."""
+    bias, se = _bias(cuda, M, N, K, dtypes.float16, layout)
+    assert bias <= 32 * 2.0 ** -22 + 4 * se, bias
