@@ -112,13 +112,21 @@ int gemm_inject_status(anl_device* dev, int code, int counter_value) {
     return ANL_OK;
 }
 
-// Is this f16 contraction worth a tensor-core launch instead of the generated one-group-of-lanes-per-output kernel?
+// Is this f16 contraction worth a tensor-core launch instead of the generated kernel of lanes that share an output?
 static bool gemm_f16_worth(const GemmPlan& gp) {
     const Contraction& c = gp.c;
     const bool padded = gp.pad_a || gp.pad_b;
     if (!padded && c.M >= 64 && c.N >= 64 && c.K >= 32) return true;
+    // A handful of outputs: a tile has eight CTAs at most, the generated reduction is split over the whole machine, and adds in
+    // f32 with rounding.  Tensor cores against generated kernel in us (K at 16384 / 262144): 64 outputs 17 / 145 against 8 / 12,
+    // 256 outputs 16 / 145 against 10 / 25, 1024 outputs 18 / 148 against 10 / 76 with both operands k-contiguous; with neither,
+    // 1024 outputs are 27 / 148 against 20 / 180, and from 4096 on the tensor cores are ahead (20 / 148 against 20 / 221 and
+    // 27 / 150 against 41 / 804).
+    if (c.M * c.N <= 1024) return false;
     // Few rows or few columns: most of a 128-row tile is empty, so it takes enough work to pay for the launch;
-    // with an operand that has to be copied first, more.
+    // with an operand that has to be copied first, more.  The generated kernel adds these sums in f32 with rounding, tensor
+    // memory cuts them, in chunks of at most 1024 terms: 5.6e-6 of a sum of positive terms, a twenty-fifth of what the one
+    // rounding to f16 leaves (1.4e-4 rms).
     const double work = (double)c.M * (double)c.N * (double)c.K;
     return c.K >= 64 && work >= (padded ? 1 << 23 : 1 << 20);
 }

@@ -117,3 +117,19 @@ def test_long_f16_sums_lose_no_more_than_one_chunk(cuda, M, N, K, layout):
     total on average, so 32 x 2^-22 in all, below the 2^-12 of the one rounding to f16."""
     bias, se = _bias(cuda, M, N, K, dtypes.float16, layout)
     assert bias <= 32 * 2.0 ** -22 + 4 * se, bias
+
+
+@pytest.mark.parametrize("M,N,K,layout", [(8, 8, 1 << 18, "KK"), (1, 64, 65536, "KK"), (10, 10, 40001, "MM"), (32, 32, 70000, "MK")])
+def test_a_handful_of_outputs_is_split_over_the_machine(cuda, M, N, K, layout):
+    """At most 1024 outputs stay with the generated reduction, in blocks that share each of them and add in f32 with rounding: sums
+    of positive terms are the rounding to f16 (2^-11) away from float64, and at most a hundredth of it more."""
+    gen = np.random.default_rng(M * N)
+    am, bm = ((gen.uniform(1, 2, (rows, K)) * np.sqrt(2000 / (2.25 * K))).astype(np.float16).astype(np.float32) for rows in (M, N))
+    a = Tensor.new_leaf((M, K), dtypes.float16).set_data(am.reshape(-1)) if layout[0] == "K" else Tensor.new_leaf((K, M), dtypes.float16).set_data(am.T.reshape(-1)).permute((1, 0))
+    b = Tensor.new_leaf((N, K), dtypes.float16).set_data(bm.reshape(-1)).permute((1, 0)) if layout[1] == "K" else Tensor.new_leaf((K, N), dtypes.float16).set_data(bm.T.reshape(-1))
+    items, ids, inputs = schedule([a.matmul(b)])
+    before = cuda.stats()["gemm_launched"]
+    y = cuda.run(items, inputs)[ids[0]].reshape(M, N)
+    assert cuda.stats()["gemm_launched"] == before
+    ref = am.astype(np.float64) @ bm.astype(np.float64).T
+    assert np.abs(y / ref - 1.0).max() <= 1.01 * 2.0 ** -11
