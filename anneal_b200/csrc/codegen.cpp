@@ -250,7 +250,7 @@ struct Gen {
             }
             if (ok && !key.empty() && prod <= 128) by_set[key].push_back(i);
         }
-        struct Cand { std::vector<int> ranges; double score; };
+        struct Cand { std::vector<int> ranges; double score, frac; };
         std::vector<Cand> outs;
         for (auto& kv : by_set) {
             if (kv.second.size() < 4) continue;
@@ -269,16 +269,28 @@ struct Gen {
             }
             bool all_out = true;
             for (int r : kv.first) if (std::find(loop_ranges.begin(), loop_ranges.end(), r) == loop_ranges.end()) all_out = false;
-            if (all_out) outs.push_back(Cand{kv.first, (double)kv.second.size() * (1.0 - frac)});
+            if (all_out) outs.push_back(Cand{kv.first, (double)kv.second.size() * (1.0 - frac), frac});
         }
         std::sort(outs.begin(), outs.end(), [](const Cand& x, const Cand& y) { return x.score > y.score; });
         std::set<int> chosen; int64_t prod = 1;
+        double off = 0;            // share of the guards that a case decides against; a slice has two
         for (auto& c : outs) {
             int64_t p2 = prod;
             for (int r : c.ranges) if (!chosen.count(r)) p2 *= N(r).arg;
             if (p2 > 128) continue;
             for (int r : c.ranges) chosen.insert(r);
-            prod = p2;
+            prod = p2; off = std::max(off, 1.0 - c.frac);
+        }
+        // Without a REDUCE the switch has to be paid for by the terms that it leaves out, and neighbouring threads must share
+        // the case, or a warp walks through all of them.  16384 x p x 8, a concatenation of p pieces, in us, guarded loads against
+        // switch: p = 4 6.1 / 8.2, 8 10.2 / 10.2, 16 20.5 / 14.3, 64 199 / 51; with the pieces along the last range 65536 x 2p
+        // 6.1 / 10.2, 10.2 / 16.4, 18.4 / 43, 201 / 168; with 4 elements behind it a scatter of 72 terms 7.4 / 8.2.
+        if (reduces.empty()) {
+            int64_t behind = 1;
+            for (size_t r = loop_ranges.size(); r-- > 0 && !chosen.count(loop_ranges[r]);) behind *= N(loop_ranges[r]).arg;
+            int loads = 0;
+            for (int i = 0; i < n; i++) if (N(i).op == OP_INDEX && i != dst && is_live(i)) loads++;
+            if (loads * off < 6.0 || behind < 8) return;
         }
         for (int r : loop_ranges) if (chosen.count(r)) enum_out.push_back(r);
     }
