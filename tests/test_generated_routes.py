@@ -25,8 +25,8 @@ def _pieces(shape, axis, count, terms=1):
 
 
 # few pieces; pieces along the last range, where neighbouring threads are in different ones; four elements behind the range |
-# many pieces; a convolution's patches (nine terms a channel); eight elements behind the range
-CASES = [((64, 32), 1, 4, 1, False), ((100, 1, 8), 1, 8, 1, False), ((500, 2), 1, 16, 1, False), ((32, 1, 4), 1, 8, 9, False),
+# many pieces; a convolution's patches (several terms a channel); eight elements behind the range
+CASES = [((64, 32), 1, 4, 1, False), ((100, 1, 8), 1, 8, 1, False), ((500, 2), 1, 16, 1, False), ((32, 1, 4), 1, 8, 4, False),
          ((9, 1, 8), 1, 16, 1, True), ((3, 1, 49), 1, 4, 9, True), ((1, 300), 0, 24, 1, True)]
 
 
