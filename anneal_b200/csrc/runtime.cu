@@ -427,16 +427,22 @@ int launch_sgd(anl_device* dev, anl_buffer* master, anl_buffer* param, anl_buffe
 // batch 64 (eight leaves and five outputs, 1 MB in all) went from 370 to 208 us, with the parsed schedule kept as well.  Above it the staging copy costs more than the calls.
 constexpr size_t kHostStageMax = (size_t)8 << 20;
 
-// the pinned block; every call that fills it waits for the stream before it returns, so it is free at the next
-static int host_stage(anl_device* dev, size_t bytes, char** out) {
-    if (dev->host_stage_bytes < bytes) {
-        if (dev->host_stage) { cudaStreamSynchronize(dev->stream); cudaFreeHost(dev->host_stage); dev->host_stage = nullptr; dev->host_stage_bytes = 0; }
-        size_t want = (size_t)1 << 18;
-        while (want < bytes) want *= 2;
-        if (cudaMallocHost(&dev->host_stage, want) != cudaSuccess) { dev->host_stage = nullptr; return dev->fail(ANL_ERR_LIMIT, "cuda: cannot allocate the pinned staging block"); }
-        dev->host_stage_bytes = want;
+// Makes the pinned block hold `bytes`, before a call queues anything of its own: every call that fills the block waits for
+// the stream before it returns, so it is free then, and what earlier calls left queued (replays, with their
+// collectives) is waited for under the watchdog.  Without the memory the block stays as it is, and the copies go the way that
+// larger ones go.
+static int reserve_host_stage(anl_device* dev, size_t bytes) {
+    if (bytes == 0 || bytes > kHostStageMax || dev->host_stage_bytes >= bytes) return ANL_OK;
+    size_t want = (size_t)1 << 18;
+    while (want < bytes) want *= 2;
+    if (dev->host_stage) {
+        if (int rc = wait_stream_watched(dev, dev->stream, "staging")) return rc;
+        cudaFreeHost(dev->host_stage);
+        dev->host_stage = nullptr; dev->host_stage_bytes = 0;
     }
-    *out = (char*)dev->host_stage;
+    if (cudaMallocHost(&dev->host_stage, dev->refuse_host_stage ? (size_t)1 << 60 : want) == cudaSuccess) { dev->host_stage_bytes = want; return ANL_OK; }
+    cudaGetLastError();                       // handled here: the next launch must not report it
+    dev->host_stage = nullptr;
     return ANL_OK;
 }
 
@@ -513,6 +519,17 @@ struct Table {
     std::unordered_map<uint32_t, anl_output> after;   // output id → placed entry asking for an all-reduce and/or an SGD update
 };
 
+// bytes of the outputs that go to host memory, each on a 64-byte boundary
+size_t host_output_bytes(Table& t, const anl_output* placed, int n_placed) {
+    size_t bytes = 0;
+    for (uint32_t id : t.finals) {
+        bool resident = false;
+        for (int k = 0; k < n_placed; k++) if (placed[k].uop_idx == id && placed[k].resident) resident = true;
+        if (!resident) bytes += ((size_t)std::max<int64_t>(t.bufs[id].elems, 0) * 4 + 63) & ~(size_t)63;
+    }
+    return bytes;
+}
+
 int build_table(anl_device* dev, const std::vector<Item>& items, const Bindings& binds,
                 const anl_input* inputs, int n_inputs, const anl_output* placed, int n_placed, Table& t) {
     for (auto& it : items) { t.written.insert(it.bufs[0].id); for (size_t b = 1; b < it.bufs.size(); b++) t.read.insert(it.bufs[b].id); }
@@ -561,10 +578,14 @@ int build_table(anl_device* dev, const std::vector<Item>& items, const Bindings&
                 leaf_bytes += ((size_t)elems * 4 + 255) & ~(size_t)255;
             }
     }
+    // final outputs: never read again, or read again but deliberately left un-aliased by the planner
+    for (auto& it : items) if (!t.read.count(it.bufs[0].id) || it.bufs[0].slot < 0) t.finals.push_back(it.bufs[0].id);
+    const bool together = leaves.size() >= 2 && leaf_bytes <= kHostStageMax;
+    const size_t out_bytes = host_output_bytes(t, placed, n_placed);
+    if (int rc = reserve_host_stage(dev, std::max(together ? leaf_bytes : 0, out_bytes <= kHostStageMax ? out_bytes : 0))) return rc;
     char* leaf_block = nullptr;
-    if (leaves.size() >= 2 && leaf_bytes <= kHostStageMax) {
-        char* stage = nullptr;
-        if (int rc = host_stage(dev, leaf_bytes, &stage)) return rc;
+    if (together && leaf_bytes <= dev->host_stage_bytes) {
+        char* const stage = (char*)dev->host_stage;
         if (int rc = dev->alloc(leaf_bytes, (void**)&leaf_block)) return rc;
         t.owned.push_back(leaf_block);
         for (const Leaf& l : leaves) { std::memcpy(stage + l.at, l.data, l.bytes); dev->stats.h2d_bytes += l.bytes; }
@@ -597,8 +618,6 @@ int build_table(anl_device* dev, const std::vector<Item>& items, const Bindings&
             t.bufs[bd.id] = d;
         }
     }
-    // final outputs: never read again, or read again but deliberately left un-aliased by the planner
-    for (auto& it : items) if (!t.read.count(it.bufs[0].id) || it.bufs[0].slot < 0) t.finals.push_back(it.bufs[0].id);
     return ANL_OK;
 }
 
@@ -984,14 +1003,8 @@ int collect_outputs(anl_device* dev, Table& t, const anl_output* placed, int n_p
     // small outputs for the host land in the pinned block and are handed out after the one wait
     struct Late { float* to; const char* from; size_t bytes; };
     std::vector<Late> late;
-    char* stage = nullptr;
-    size_t stage_bytes = 0;
-    for (uint32_t id : t.finals) {
-        bool resident = false;
-        for (int k = 0; k < n_placed; k++) if (placed[k].uop_idx == id && placed[k].resident) resident = true;
-        if (!resident) stage_bytes += ((size_t)std::max<int64_t>(t.bufs[id].elems, 0) * 4 + 63) & ~(size_t)63;
-    }
-    if (stage_bytes > 0 && stage_bytes <= kHostStageMax) { if (host_stage(dev, stage_bytes, &stage) != ANL_OK) stage = nullptr; }
+    const size_t stage_bytes = host_output_bytes(t, placed, n_placed);
+    char* const stage = stage_bytes <= std::min(kHostStageMax, dev->host_stage_bytes) ? (char*)dev->host_stage : nullptr;
     size_t stage_at = 0;
     for (uint32_t id : t.finals) {
         if (n >= cap) { rc = dev->fail(ANL_ERR_LIMIT, "run: more final outputs than the caller made room for"); break; }
@@ -1167,6 +1180,16 @@ int anl_gemm_inject_status(anl_device* dev, int code, int counter_value) {
     if (!dev) return ANL_ERR_INVALID;
     cudaSetDevice(dev->ordinal);
     return gemm_inject_status(dev, code, counter_value);
+}
+
+int anl_inject_host_stage_failure(anl_device* dev, int on) {
+    if (!dev) return ANL_ERR_INVALID;
+    cudaSetDevice(dev->ordinal);
+    if (int rc = wait_stream_watched(dev, dev->stream, "staging")) return rc;
+    if (dev->host_stage) cudaFreeHost(dev->host_stage);
+    dev->host_stage = nullptr; dev->host_stage_bytes = 0;
+    dev->refuse_host_stage = on != 0;
+    return ANL_OK;
 }
 
 void* anl_stream(anl_device* dev) { return dev ? (void*)dev->stream : nullptr; }
@@ -1661,6 +1684,7 @@ static int graph_replay_impl(anl_graph* g, const anl_input* inputs, int n_inputs
         dev->stats.graph_captures++;
     } else {
         // replay: refresh host-fed leaves in place
+        rc = reserve_host_stage(dev, host_output_bytes(g->table, placed, n_placed));
         for (int k = 0; k < n_inputs && rc == ANL_OK; k++) {
             if (inputs[k].resident || !inputs[k].data) continue;
             host_fed = true;

@@ -148,6 +148,7 @@ struct anl_device {
     static constexpr size_t kMaxSchedules = 8;
     void* host_stage = nullptr;           // pinned: small host-fed runs move all leaves, and all outputs, through it
     size_t host_stage_bytes = 0;
+    bool refuse_host_stage = false;       // anl_inject_host_stage_failure
     int* gemm_status_host = nullptr;      // mapped, host-visible: code of a barrier wait that ran out
     int* gemm_status_dev = nullptr;
     std::unordered_map<std::string, void*> pair_kernels;   // configuration (tunables + fused consumer's text) -> loaded two-CTA kernel

@@ -299,6 +299,10 @@ int anl_gemm_set_defaults(anl_device* dev, const int* opts);
  * again.  No counterpart in the reference. */
 int anl_gemm_inject_status(anl_device* dev, int code, int counter_value);
 
+/* Diagnostic: with `on` non-zero the device gives up the pinned block that small host-fed runs go through, and asks
+ * for one that no host can give it from then on; such runs must then work by separate copies. */
+int anl_inject_host_stage_failure(anl_device* dev, int on);
+
 /* The cudaStream_t this device queues its kernels and copies on (non-blocking: it is not ordered
  * with the default stream).  A caller that launches work of its own on device buffers — through
  * anl_sum_f32_static, say — passes this handle to stay in order with uploads, runs and downloads;

@@ -3,6 +3,7 @@ below the size that is staged, f16 leaves beside f32 ones."""
 import numpy as np
 import pytest
 
+from anneal_b200.device import Device
 from anneal_b200.tensor import Tensor
 from anneal_b200.uop import dtypes
 from util import schedule
@@ -42,3 +43,26 @@ def test_half_leaves_and_many_schedules(cuda, oracle):
             got, want = cuda.run(items, inputs), oracle.run(items, inputs)
             for i in ids:
                 assert np.array_equal(got[i], want[i])
+
+
+def test_runs_go_on_without_the_pinned_block():
+    """The host may have no pinned memory left: the copies then go one by one, and the refusal is not reported by a later
+    launch (an f16 output is converted by a kernel before its copy)."""
+    dev = Device(0)
+    try:
+        plain, half = _product(1000, 3), _product(1000, 4, dtypes.float16)
+        before = [dev.run(items, inputs) for items, _, inputs in (plain, half)]
+        dev._check(dev.L.anl_inject_host_stage_failure(dev.h, 1))
+        for _ in range(2):
+            for (items, ids, inputs), want in zip((plain, half), before):
+                got = dev.run(items, inputs)
+                for i in ids:
+                    assert np.array_equal(got[i], want[i])
+                got = dev.replay(items, inputs)
+                for i in ids:
+                    assert np.array_equal(got[i], want[i])
+        dev._check(dev.L.anl_inject_host_stage_failure(dev.h, 0))
+        got = dev.run(plain[0], plain[2])
+        assert all(np.array_equal(got[i], before[0][i]) for i in plain[1])
+    finally:
+        dev.close()
