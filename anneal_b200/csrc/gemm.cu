@@ -524,10 +524,10 @@ int gemm_tf32_source(const Plan& plan, std::string& out, std::string& note) {
 }
 
 // The one-CTA kernel for f32 contractions with few tiles.  Measured against the pair kernel (and the launch that adds its
-// copies up), us with the operand splits and the events: 256 x 4096 x 1024 31.7 / 35.8, 64 x 4096 x 1024 25.6 / 31.7,
-// 100 x 1000 x 700 17.4 / 29.7, 600-cubed 19.5 / 29.7, 1024-cubed 29.7 / 34.8, 512 x 4096 x 1024 39.9 / 46.1, 2048 x 1024 x 1024
-// 39.9 / 46.1 (32 tiles), 1024 x 1024 x 2048 44.0 / 46.0, 300 x 1024 x 4096 44.1 / 44.0; the other way 256 x 1024 x 4096 42.0 / 37.9
-// and 40 x 1024 x 4096 37.9 / 31.7 (the pair kernel has 16 slices where a cluster has 4), 1024 x 4096 x 1024 (64 tiles) and
+// copies up), us with the operand splits and the events: 256 x 4096 x 1024 29.7 / 35.8, 64 x 4096 x 1024 25.6 / 31.7,
+// 100 x 1000 x 700 17.4 / 29.7, 600-cubed 19.5 / 29.7, 1024-cubed 27.6 / 34.8, 512 x 4096 x 1024 39.9 / 46.1, 2048 x 1024 x 1024
+// 37.9 / 46.1 (32 tiles), 1024 x 1024 x 2048 42.0 / 46.0, 300 x 1024 x 4096 44.0 / 44.0; the other way 256 x 1024 x 4096 39.9 / 37.9
+// and 40 x 1024 x 4096 35.8 / 31.7 (the pair kernel has 16 slices where a cluster has 4), 1024 x 4096 x 1024 (64 tiles) and
 // 1024 x 1024 x 8192 198 / 126.  Its error is no larger there: chunks of 256 terms, where the pair kernel takes 256 to 1024.
 static bool tf32_small_takes(int64_t M, int64_t N, int64_t K) {
     const int64_t tiles = ((M + 255) / 256) * ((N + 255) / 256);

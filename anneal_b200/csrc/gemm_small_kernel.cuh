@@ -26,8 +26,8 @@
 // more warps than the two that load and multiply take each finished chunk to registers and add it to the ones before, in f32
 // round-to-nearest, while the next one is multiplied.  Error against float64 (rms with normal values | mean with positive
 // ones), slices of 1024 f32 terms in one go, in chunks of 256, on the pair kernel: 256 x 1024 x 4096 7.1e-6 | 1.1e-5, 1.7e-6 |
-// 2.3e-6, 1.7e-6 | 2.3e-6 (37.9, 42.0, 37.9 us alone, with the operand splits and the events); 2048 x 1024 x 1024 7.1e-6 | 1.1e-5,
-// 1.7e-6 | 2.3e-6, 3.5e-6 | 5.1e-6 (35.8, 39.9, 46.1 us).  Eight f16 slices of 8192 terms lost 4.7e-5 of a positive sum, in chunks
+// 2.3e-6, 1.7e-6 | 2.3e-6 (37.9, 39.9, 37.9 us alone, with the operand splits and the events); 2048 x 1024 x 1024 7.1e-6 | 1.1e-5,
+// 1.7e-6 | 2.3e-6, 3.5e-6 | 5.1e-6 (35.8, 37.9, 46.1 us).  Eight f16 slices of 8192 terms lost 4.7e-5 of a positive sum, in chunks
 // of 1024 they lose 5.6e-6, beside the 1.4e-4 rms of the rounding to f16 (40 x 4096 x 16384 34.8 and 38.9 us).
 //
 // With fewer than 128 rows only CFG_PROWS of them are loaded and staged; the MMA still reads 128 rows of
@@ -147,7 +147,10 @@ gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_con
 gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_constant__ TensorMap map_b, const SmallGemmArgs g) {
 #endif
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) unsigned long long full_bar[NSTAGE], empty_bar[NSTAGE], acc_full[2], acc_empty[2];
+    __shared__ __align__(8) unsigned long long full_bar[NSTAGE], empty_bar[NSTAGE], acc_full[CHUNK ? 2 : 1];
+#if CFG_CHUNK
+    __shared__ __align__(8) unsigned long long acc_empty[2];
+#endif
     __shared__ unsigned tmem_base_slot;
     __shared__ volatile int failed;
 
@@ -163,7 +166,11 @@ gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_con
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < NSTAGE; s++) { mbar_init(smem_u32(&full_bar[s]), 1); mbar_init(smem_u32(&empty_bar[s]), 1); }
-        for (int a = 0; a < 2; a++) { mbar_init(smem_u32(&acc_full[a]), 1); mbar_init(smem_u32(&acc_empty[a]), 8); }
+        mbar_init(smem_u32(&acc_full[0]), 1);
+#if CFG_CHUNK
+        mbar_init(smem_u32(&acc_full[1]), 1);
+        for (int a = 0; a < 2; a++) mbar_init(smem_u32(&acc_empty[a]), 8);
+#endif
         failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -228,20 +235,28 @@ gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_con
             const unsigned idesc = (1u << 4) | ((CFG_TF32 ? 2u : 0u) << 7) | ((CFG_TF32 ? 2u : 0u) << 10) | ((CFG_A_MN ? 1u : 0u) << 15) | ((CFG_B_MN ? 1u : 0u) << 16) | ((unsigned)(NT >> 3) << 17) | ((unsigned)(BM >> 4) << 24);
             unsigned stage = 0, phase = 0;
             bool ok = true;
-            for (int it = 0; it < nkb; it++) {
+#if CFG_CHUNK
+            // chunk ch has accumulator ch & 1, which the chunk two before it has to have left
+            for (int ch = 0, first = 0; first < nkb && ok; ch++, first += CHUNK) {
+            if (!mbar_wait(smem_u32(&acc_empty[ch & 1]), ((unsigned)(ch >> 1) & 1u) ^ 1u, &failed)) { ok = false; *(volatile int*)g.status = 24; break; }
+            const int end = first + CHUNK < nkb ? first + CHUNK : nkb;
+#else
+            constexpr int ch = 0, first = 0;
+            const int end = nkb;
+            {
+#endif
+            const unsigned acc = tmem_base + (ch & 1) * NT;
+            for (int it = first; it < end; it++) {
                 if (!mbar_wait(smem_u32(&full_bar[stage]), phase, &failed)) { ok = false; *(volatile int*)g.status = 22; break; }
-                // chunk ch has accumulator ch & 1, which the chunk two before it has to have left
-                const int ch = CHUNK ? it / (CHUNK ? CHUNK : 1) : 0, kc = it - ch * CHUNK;
-                if (CHUNK && kc == 0 && !mbar_wait(smem_u32(&acc_empty[ch & 1]), ((unsigned)(ch >> 1) & 1u) ^ 1u, &failed)) { ok = false; *(volatile int*)g.status = 24; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const unsigned sp = smem_base + stage * STAGE_BYTES, sq = sp + P_BYTES, acc = tmem_base + (ch & 1) * NT;
+                const unsigned sp = smem_base + stage * STAGE_BYTES, sq = sp + P_BYTES;
 #if CFG_TF32
                 // A_lo · B_hi, A_hi · B_lo, A_hi · B_hi
 #pragma unroll
                 for (int pass = 0; pass < 3; pass++) {
                     const unsigned pp = pass == 0 ? sp + P_PART : sp, pq = pass == 1 ? sq + Q_PART : sq;
 #pragma unroll
-                    for (int k = 0; k < 4; k++) umma_f16(acc, make_desc(pp + k * 32, 16, 1024), make_desc(pq + k * 32, 16, 1024), idesc, (kc | pass | k) != 0);
+                    for (int k = 0; k < 4; k++) umma_f16(acc, make_desc(pp + k * 32, 16, 1024), make_desc(pq + k * 32, 16, 1024), idesc, it != first || (pass | k) != 0);
                 }
 #else
 #pragma unroll
@@ -250,14 +265,15 @@ gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_con
                     // 128 bytes, 64-wide m/n groups one box apart.
                     const unsigned long long ad = CFG_A_MN ? make_desc(sp + k * 2048, BK * 128, 1024) : make_desc(sp + k * 32, 16, 1024);
                     const unsigned long long bd = CFG_B_MN ? make_desc(sq + k * 2048, BK * 128, 1024) : make_desc(sq + k * 32, 16, 1024);
-                    umma_f16(acc, ad, bd, idesc, (kc | k) != 0);
+                    umma_f16(acc, ad, bd, idesc, it != first || k != 0);
                 }
 #endif
                 umma_commit(smem_u32(&empty_bar[stage]));
-                if (it + 1 == nkb || (CHUNK && kc + 1 == CHUNK)) umma_commit(smem_u32(&acc_full[ch & 1]));
                 if (++stage == NSTAGE) { stage = 0; phase ^= 1; }
             }
-            if (!ok) failed = 1;
+            if (ok) umma_commit(smem_u32(&acc_full[ch & 1]));
+            else failed = 1;
+            }
         }
     }
     __syncwarp();
