@@ -488,6 +488,7 @@ struct Gen {
     std::map<std::pair<int, int>, std::string> memo;   // (node, ctx) → expression
     int vec_range = -1;                     // loop variable unrolled by the vector path, or -1
     std::map<int, std::string> vec_load;    // INDEX node → array name holding V preloaded values
+    int split_parts = 1;                    // blocks an output (-1: counted at launch)
     bool split_mode = false;                // every output's REDUCE is shared by SPLIT blocks (build_reduce)
     int reduce_vec = 1;                     // consecutive elements a lane takes per trip of the innermost reduce range
     std::string reduce_combine_mode;        // set by the kernel builder
@@ -891,12 +892,16 @@ struct Gen {
 
     // Trips of a reduce loop whose loads the compiler may issue together: eight for a short body, fewer where the
     // copies would bloat the kernel, never more than a lane makes.  The additions stay in order.  Without it each trip
-    // waits for its own loads: a column sum over 64 rows by four lanes took 9.2 us (16 dependent trips), now 3.3.
+    // waits for its own loads: a column sum over 64 rows by four lanes took 9.2 us (16 dependent trips), now 3.3.  From 32
+    // trips on the compiler's own choice is better (65536 x 1024 f32 summed over the rows 178 us eight at a time, 60 so; 8192 x 8192
+    // f16 46 and 37), and where the parts are counted at launch a lane makes as many.
     std::string loop_unroll(int red, int64_t terms) {
         const int64_t lines = (int64_t)std::count(loop[red].code.begin(), loop[red].code.end(), '\n');
         int64_t u = lines <= 12 ? 8 : lines <= 30 ? 4 : lines <= 60 ? 2 : 1;
         if (!enum_out.empty()) u = 1;           // a copy per case already: 72 cases unrolled four times ran 37.7 us instead of 22.6, from instruction memory
         if (terms > 0) while (u > 1 && u * lanes > terms) u /= 2;
+        if (split_parts > 1) terms /= split_parts;
+        if (terms >= (int64_t)lanes * 32 || split_parts < 0) u = 1;
         return u > 1 ? "_Pragma(\"unroll " + std::to_string(u) + "\") " : std::string();
     }
 
@@ -1853,9 +1858,14 @@ struct Gen {
         };
         if (dyn) { int64_t l, t; split_layout(l, t); lanes = (int)l; touts = (int)t; }
 
-        // Split one long reduction over several blocks?  Where the outputs alone leave SMs idle, and a lane keeps
-        // at least 16 terms (4 wide loads): below that the ticket and the second pass over the partials, about
-        // 1.5 us, cost what the shorter loop saves.  One launch instead of a partials and a finish kernel, whose
+        // Split one long reduction over several blocks?  Where the outputs alone leave SMs idle (fewer than 256 blocks) and a
+        // lane makes more than 64 trips: below that the ticket and the second pass over the partials cost what the shorter loop
+        // saves.  us split / in one piece: f32 sums of 128 x 128 (64 trips) 3.2 / 2.2, 256 x 256 3.2 / 5.0; over the
+        // rows of 1024 x 1024 3.9 / 2.5, 256 x 1024 3.5 / 1.9, 8192 x 8192 (1024 blocks) 52.8 / 47.6, 8192 x 1000 (125 blocks)
+        // 10.7 / 14.4, 65536 x 1024 60 / 107.  Each part keeps at least 16 terms a lane (4 wide loads), and the cases of a switch,
+        // whose trips are long, are split from there on (a CNN step's weight gradient with 98 trips a lane: the step 76 us split,
+        // 87 in one piece).
+        // One launch instead of a partials and a finish kernel, whose
         // serial last sum took 2 to 7 us: the loss sum over 8192 x 1000 f16 terms 25 + 6.8 us before.  Over the
         // bound batch, against one block (or one thread) per output: the squared-error sum over 65536 x 1024 f32
         // terms took 167 ms and the column sums of a 65536 x 4096 matrix 3.67 ms; together they are now under
@@ -1868,7 +1878,8 @@ struct Gen {
                 split_layout(lanes_s, touts_s);
                 const int64_t nob = (total + touts_s - 1) / touts_s;
                 const int64_t s = std::min<int64_t>(rmax / (lanes_s * 16), (148 * 4) / nob);
-                if (s > 1 && nob <= 148 * 2) { split = (int)std::min<int64_t>(s, 1024); lanes = (int)lanes_s; touts = (int)touts_s; }
+                const bool long_loop = rmax > (int64_t)lanes * 64 && (total + touts - 1) / touts < 256;
+                if (s > 1 && (enum_out.empty() ? long_loop : nob <= 148 * 2)) { split = (int)std::min<int64_t>(s, 1024); lanes = (int)lanes_s; touts = (int)touts_s; }
             }
             if (split > 1 && opts.split > 1) { rc_layout = true; lanes = threads; touts = 1; }
             if (split > 1 && (total + touts - 1) / touts > kMaxTickets) split = 1;
@@ -1879,6 +1890,7 @@ struct Gen {
         // no cooperation at all (one lane per output) or one output per block
         if (!enum_out.empty() && !((lanes == 1 && split == 1) || touts == 1)) enum_out.clear();
         split_mode = split != 1;
+        split_parts = split;
 
         reset_emit();
         reduce_combine_mode = "group";
