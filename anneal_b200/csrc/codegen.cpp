@@ -488,6 +488,10 @@ struct Gen {
     std::map<std::pair<int, int>, std::string> memo;   // (node, ctx) → expression
     int vec_range = -1;                     // loop variable unrolled by the vector path, or -1
     std::map<int, std::string> vec_load;    // INDEX node → array name holding V preloaded values
+    // A row's reduction and then a sweep over it in one kernel (build_rowbcast): with wide loads or an unroll count on the
+    // reduction the compiler leaves the sweep, which is the longer part, without its own unrolling (100000 values in one
+    // block 37 us as it is, 80 with wide loads; 4096 rows of 9000 90 and 116).
+    bool row_broadcast = false;
     int split_parts = 1;                    // blocks an output (-1: counted at launch)
     bool split_mode = false;                // every output's REDUCE is shared by SPLIT blocks (build_reduce)
     int reduce_vec = 1;                     // consecutive elements a lane takes per trip of the innermost reduce range
@@ -869,7 +873,7 @@ struct Gen {
     // Only where lanes run along the reduce range (RC layout), the range is static and a multiple of the
     // width, and at least one operand then arrives by 128-bit loads.
     int pick_reduce_vec(int red, const std::vector<int>& rr) {
-        if (!rc_layout || rr.empty() || unroll_short_loops || opts.debug_bounds || opts.vector_width == 1 || enum_reduce.count(red)) return 1;
+        if (!rc_layout || rr.empty() || unroll_short_loops || row_broadcast || opts.debug_bounds || opts.vector_width == 1 || enum_reduce.count(red)) return 1;
         const int last = rr.back();
         if (N(last).symbolic() || N(last).arg < 64) return 1;
         const int keep = chain_vec;
@@ -897,6 +901,7 @@ struct Gen {
     // f16 46 and 37), and where the parts are counted at launch a lane makes as many.
     std::string loop_unroll(int red, int64_t terms) {
         const int64_t lines = (int64_t)std::count(loop[red].code.begin(), loop[red].code.end(), '\n');
+        if (row_broadcast) return std::string();
         int64_t u = lines <= 12 ? 8 : lines <= 30 ? 4 : lines <= 60 ? 2 : 1;
         if (!enum_out.empty()) u = 1;           // a copy per case already: 72 cases unrolled four times ran 37.7 us instead of 22.6, from instruction memory
         if (terms > 0) while (u > 1 && u * lanes > terms) u /= 2;
@@ -1798,6 +1803,7 @@ struct Gen {
         std::ostringstream k;
         k << reduce_macros() << preamble();
         std::string name = "reduce_rowbcast";
+        row_broadcast = true;
         k << signature(name, false, threads) << " {\n  enter_();\n";
         k << "  __shared__ float red_smem[" << std::max(threads / 32, 1) << "];\n";
         k << "  const int lane = threadIdx.x, grp = 0;\n";
