@@ -4,6 +4,7 @@ import pytest
 
 import util_chains as C
 from anneal_b200.device import lower_chain
+from anneal_b200.tensor import Tensor
 from util import rel_err
 
 
@@ -36,6 +37,17 @@ def test_whole_row_over_its_own_operand_stays_a_chain():
     items, _, _ = C.plan(C.row_over_operand(70, 300))
     assert C.slots(items) == [0, 1, 0, -1]
     assert "2 stages" in lower_chain(items, 1, 2)["note"]
+
+
+def test_vectors_alone_are_no_chain():
+    """Kernels of one value a row with nothing to run along it are elementwise kernels, a thread a value."""
+    leaf = lambda n: Tensor.new_leaf((n,)).set_data(np.ones(n, np.float32))
+    items, _, _ = C.plan([v.mul(v) for v in (leaf(1000), leaf(1000), leaf(1000))])
+    with pytest.raises(Exception, match="runs along the row"):
+        lower_chain(items, 0, 3)
+    x, v = Tensor.new_leaf((300, 40)).set_data(np.ones(12000, np.float32)), leaf(300)
+    items, _, _ = C.plan([x.sum((1,)).mul(v), v.mul(v)])
+    assert "2 stages" in lower_chain(items, 0, 2)["note"]
 
 
 @pytest.mark.gpu
