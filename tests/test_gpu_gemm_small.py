@@ -133,3 +133,24 @@ def test_a_handful_of_outputs_is_split_over_the_machine(cuda, M, N, K, layout):
     assert cuda.stats()["gemm_launched"] == before
     ref = am.astype(np.float64) @ bm.astype(np.float64).T
     assert np.abs(y / ref - 1.0).max() <= 1.01 * 2.0 ** -11
+
+
+@pytest.mark.parametrize("batch,width,out", [(257, 4104, 264), (256, 12288, 136)])
+def test_fused_consumer_behind_chunks(cuda, oracle, batch, width, out):
+    """A layer whose slices of K are longer than a chunk, with its bias and GELU in the epilogue."""
+    from anneal_b200.device import lower_gemm
+    x, layers = hleaf((batch, width), 5), [nn.Linear(width, out, True, dtypes.float16), nn.Linear(out, 72, True, dtypes.float16)]
+    for k, l in enumerate(layers):
+        for p in l.params():
+            p.value[:] = W.normal(33, k, p.value.size) * np.float32(0.05)
+            p.load()
+    y = layers[1].forward(nn.gelu_tanh(layers[0].forward(x)))
+    R.MATERIALIZE_CONTRACTION_OPERANDS = "auto"
+    try:
+        source = lower_gemm(schedule([y])[0], 0, fuse_next=True)["source"]
+        assert "#define CFG_CHUNK 16\n" in source and "#define CFG_EPI 1\n" in source
+        before = cuda.stats()["epilogues_fused"]
+        compare(cuda, oracle, [y], F16, what=f"chunks {batch}x{width}")
+    finally:
+        R.MATERIALIZE_CONTRACTION_OPERANDS = False
+    assert cuda.stats()["epilogues_fused"] > before
