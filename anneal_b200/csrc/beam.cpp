@@ -13,8 +13,9 @@
 // A dense f16 contraction is searched too — it is where the reference's Tile / Upcast / Vectorize
 // act (codegen/opt.go:206-307, 318-556) — but over the hand-written kernel's own tunables: tile
 // width, depth of the shared-memory ring, raster group, and a flag word (1 streaming stores, 2 the
-// one-CTA kernel).  None of them changes the order of the additions inside a tile, so the guard is
-// bit-identity.
+// one-CTA kernel).  Where the one-CTA kernel takes the contraction by default, its own tile width and ring
+// depth are searched; its slices of K stay as they are.  None of these changes the order of the additions, so the guard
+// is bit-identity.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -162,10 +163,7 @@ static int beam_search_gemm(anl_device* dev, const Item& it, int width, int dept
     double base_us = 0;
     if (rc == ANL_OK) rc = run_one(base_o, &base_us, ref);
     if (rc == ANL_OK) {
-        const int tile_v[] = {256, 128};
-        const int stage_v[] = {4, 5, 6, 7};
-        const int group_v[] = {-1, 1, 2, 4, 8, 16};
-        const int flag_v[] = {1, 2};
+        const int parts = gemm_small_parts(*base_plan);
         if (width <= 0) width = 4;
         if (depth <= 0) depth = 4;
         std::vector<Cand> frontier = {Cand{{0, 0, 0, 0}, base_us}};
@@ -174,8 +172,8 @@ static int beam_search_gemm(anl_device* dev, const Item& it, int width, int dept
         for (int d = 0; d < depth; d++) {
             std::vector<Cand> next;
             for (const Cand& c : frontier) {
-                auto try_set = [&](int knob, int value) {
-                    Cand n = c; n.o[knob] = value;
+                auto try_set = [&](int knob, int value, int flags) {
+                    Cand n = c; n.o[knob] = value; n.o[3] = flags;
                     char k[64]; std::snprintf(k, sizeof k, "%d,%d,%d,%d", n.o[0], n.o[1], n.o[2], n.o[3]);
                     if (std::find(seen.begin(), seen.end(), k) != seen.end()) return;
                     seen.push_back(k);
@@ -185,10 +183,18 @@ static int beam_search_gemm(anl_device* dev, const Item& it, int width, int dept
                     n.us = us;
                     next.push_back(n);
                 };
-                for (int v : tile_v) try_set(0, v);
-                for (int v : stage_v) try_set(1, v);
-                for (int v : group_v) try_set(2, v);
-                for (int v : flag_v) try_set(3, v);
+                if (parts > 0) {
+                    for (int v : {128, 64, 32}) try_set(0, v, 2);
+                    for (int v : {2, 3, 4, 5, 6, 7, 8}) try_set(1, v, 2);
+                }
+                if (parts <= 1) {          // the pair kernel adds all of K in one go
+                    for (int v : {256, 128}) try_set(0, v, parts ? 0 : c.o[3]);
+                    if (parts == 0) {
+                        for (int v : {4, 5, 6, 7}) try_set(1, v, c.o[3]);
+                        for (int v : {-1, 1, 2, 4, 8, 16}) try_set(2, v, c.o[3]);
+                        for (int v : {1, 2}) try_set(3, v, v);
+                    }
+                }
             }
             if (next.empty()) break;
             std::sort(next.begin(), next.end(), [](const Cand& a, const Cand& b) { return a.us < b.us; });

@@ -346,7 +346,18 @@ SmallVariant choose_small(int64_t M, int64_t N, int64_t K, bool a_mn, bool b_mn,
     while (v.stages > 2 && small_smem_bytes(v) > room) v.stages--;
     return v;
 }
-SmallVariant choose_small(const GemmPlan& gp, int64_t M) { return choose_small(M, gp.c.N, gp.c.K, gp.a_mn, gp.b_mn, false); }
+SmallVariant choose_small(const GemmPlan& gp, int64_t M) {
+    SmallVariant v = choose_small(M, gp.c.N, gp.c.K, gp.a_mn, gp.b_mn, false);
+    // a search may set the tile's width and the depth of the ring; the slices of K, and with them the order of the additions, stay
+    if (!gp.tune.single_cta) return v;
+    const int nt = gp.tune.tile_n;
+    if (nt == 128 || nt == 64 || (nt == 32 && !gp.b_mn)) {
+        v.nt = nt;
+        for (v.stages = 8; v.stages > 2 && small_smem_bytes(v) > 110 * 1024;) v.stages--;
+    }
+    if (gp.tune.stages >= 2) for (v.stages = std::min(gp.tune.stages, 8); v.stages > 2 && small_smem_bytes(v) > 220 * 1024;) v.stages--;
+    return v;
+}
 
 std::string small_source(const SmallVariant& v, const std::string& epilogue) {
     std::string s;
@@ -385,6 +396,12 @@ bool small_takes(const GemmPlan& gp, int64_t M) {
 }
 
 }  // namespace
+
+int gemm_small_parts(const Plan& plan) {
+    if (!gemm_fusable(plan) || !small_takes(*plan.gemm, plan.gemm->c.M)) return 0;
+    const SmallVariant v = choose_small(*plan.gemm, plan.gemm->c.M);
+    return v.splits * (v.chunk ? 2 : 1);
+}
 
 // the source that a launch of this plan will use, and the kernel itself
 int gemm_source(anl_device* dev, const Plan& plan, const std::string& epilogue, std::string& out) {

@@ -181,8 +181,8 @@ int anl_benchmark(anl_device* dev, const uint8_t* blob, size_t blob_len, int ind
  * ANL_OPEN_BEAM applies cached winners in anl_run and searches on a miss.
  * A dense f16 contraction (routed to the tcgen05 kernels) is searched over that kernel's tunables
  * instead: `opts` is then {tile_n, stages, group_m, flags} with flags bit 0 = streaming stores,
- * bit 1 = one-CTA kernel, and the guard is bit-identity (the one-CTA kernel where it splits K reorders a sum and is
- * then rejected). */
+ * bit 1 = one-CTA kernel, and the guard is bit-identity (where the one-CTA kernel is the default, tile_n 128, 64 or 32 and
+ * stages 2 to 8 are its own, and its slices of K stay; where it is not and would split K, it is rejected). */
 typedef struct { int opts[4]; double base_us, best_us; int candidates_tried, candidates_rejected, from_cache; } anl_beam_result;
 int anl_beam_search(anl_device* dev, const uint8_t* blob, size_t blob_len, int index, int width, int depth,
                     const char* cache_path, anl_beam_result* out);

@@ -92,3 +92,26 @@ def test_contraction_search_covers_the_tensor_core_kernel(cuda, tmp_path):
     finally:
         os.environ.pop("ANNEAL_BEAM_CACHE", None)
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("rows,width,k", [(32, 1024, 4096), (300, 512, 2048)])
+def test_contraction_search_on_the_one_cta_kernel(cuda, tmp_path, monkeypatch, rows, width, k):
+    """Where the one-CTA kernel is the default, its own tile width and ring depth are searched with its slices of K as they
+    are: no candidate reorders a sum, and a device that applies the winner gives the same bits."""
+    from anneal_b200.uop import dtypes
+    rng = np.random.default_rng(4)
+    a = Tensor.new_leaf((rows, k), dtypes.float16).set_data(rng.standard_normal(rows * k) * 0.1)
+    w = Tensor.new_leaf((width, k), dtypes.float16).set_data(rng.standard_normal(width * k) * 0.1)
+    items, out_ids, inputs = schedule([a.matmul(w.permute((1, 0)))])
+    cache = str(tmp_path / "beam.json")
+    r = cuda.beam_search(items[0], cache_path=cache)
+    assert not r["from_cache"] and r["tried"] >= 10 and r["rejected"] == 0, r
+    assert r["best_us"] <= r["base_us"] * 1.0001
+    want = cuda.run(items, inputs)[out_ids[0]]
+    monkeypatch.setenv("ANNEAL_BEAM_CACHE", cache)
+    tuned = Device(0, Device.BEAM)
+    try:
+        assert np.array_equal(tuned.run(items, inputs)[out_ids[0]], want)
+        assert tuned.stats()["gemm_launched"] >= 1
+    finally:
+        tuned.close()
