@@ -2160,14 +2160,17 @@ bool render_row_chain(const std::vector<const Item*>& items, const std::vector<s
         for (auto& b : row_bufs) all32 = all32 && b.second == DT_F32;
         if (C >= 512) { if (all16 && out_bytes == 2 && C % 8 == 0) vec = 8; else if (C % 4 == 0 || all32) vec = 4; }
         shifted = C % vec != 0;
-        // elements of each operand a lane: 16, or 20 where that halves the block (4097 to 5120 elements: three blocks of 256
-        // threads an SM instead of two of 512 that a fifth of the lanes sit out)
+        // elements of each operand a lane: 16, or 20 where that halves a block of 256 to 1024 threads (rows of 2049 to 2560,
+        // 4097 to 5120 and 8193 to 10240 elements: more blocks an SM, and fewer lanes past the row's end).  us forward + backward, 16 a
+        // lane / 20: 8192 x 2052 48.7 / 39.1, 4096 x 9000 109.5 / 94.5, 4096 x 10200 114.7 / 100.5.  Not at 1024 threads,
+        // which have 64 registers each.
         const int64_t most = 16;
+        auto per_lane = [&](int l) -> int64_t { return l >= 128 && l <= 512 ? 20 : most; };
         // up to 16 elements: one thread a row, which adds them up in the reference's order, like the separate kernels do
         if (C <= most) lanes = 1;
         const int64_t span = C + (shifted ? vec - 1 : 0);
-        while (lanes < 1024 && (int64_t)lanes * (lanes == 256 ? 20 : most) < span) lanes *= 2;
-        if ((int64_t)lanes * most < span && lanes != 256) held = false;
+        while (lanes < 1024 && lanes * per_lane(lanes) < span) lanes *= 2;
+        if (lanes * per_lane(lanes) < span) held = false;
         chunks = (int)((span + (int64_t)lanes * vec - 1) / ((int64_t)lanes * vec));
         if (lanes <= 32) rows_per_block = 128 / lanes;        // a warp a row needs no barrier, so rows share a block
     }

@@ -92,3 +92,9 @@ def test_chains_that_differ_only_in_what_they_share(cuda, oracle, rows, cols, fi
     rows += 0 if first else 1
     _deviation(cuda, oracle, rows, cols, first)
     _deviation(cuda, oracle, rows, cols, not first)
+
+
+# 20 elements a lane, where that halves the block: the first and the last row length of each range, and rows that are fetched ahead
+@pytest.mark.parametrize("rows,cols", [(3, 2049), (3, 2560), (3, 2561), (2, 8193), (2, 10240), (2, 10241), (700, 2501), (700, 9001)])
+def test_rows_that_halve_the_block(cuda, oracle, rows, cols):
+    assert _softmax(cuda, oracle, rows, cols) == 1
