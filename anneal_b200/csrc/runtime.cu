@@ -197,7 +197,7 @@ int ensure_driver(anl_device* dev) {
         return e == cudaSuccess && q == cudaDriverEntryPointSuccess && *fn;
     };
     bool ok = get("cuModuleLoadData", (void**)&dev->drv.ModuleLoadData) && get("cuModuleUnload", (void**)&dev->drv.ModuleUnload) &&
-              get("cuModuleGetFunction", (void**)&dev->drv.ModuleGetFunction) && get("cuLaunchKernel", (void**)&dev->drv.LaunchKernel) &&
+              get("cuModuleGetFunction", (void**)&dev->drv.ModuleGetFunction) &&
               get("cuGetErrorString", (void**)&dev->drv.GetErrorString) && get("cuTensorMapEncodeTiled", (void**)&dev->drv.TensorMapEncodeTiled) &&
               get("cuLaunchKernelEx", (void**)&dev->drv.LaunchKernelEx) && get("cuFuncSetAttribute", (void**)&dev->drv.FuncSetAttribute);
     if (!ok) return dev->fail(ANL_ERR_CUDA, "cuda: driver entry points unavailable");
