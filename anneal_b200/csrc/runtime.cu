@@ -682,16 +682,6 @@ int try_row_chain(anl_device* dev, const std::vector<Item>& items, size_t first,
             // with its rows in registers a chain pays from one row on (one launch for several); otherwise a block a
             // row has to fill the machine
             if (!render_row_chain(members, reads, o, cp->r, err) || (rows < 128 && !cp->r.held)) cp.reset();
-            else {
-                std::shared_ptr<Module> mod;
-                if (int rc = compile_source(dev, cp->r.source, mod)) return rc;
-                CUresult cr = dev->drv.ModuleGetFunction(&cp->fn, mod->mod, cp->r.entry.c_str());
-                if (cr != CUDA_SUCCESS) return dev->fail(ANL_ERR_CUDA, "cuda: row_chain entry point missing");
-                if (cp->r.smem_bytes) {
-                    cr = dev->drv.FuncSetAttribute(cp->fn, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)cp->r.smem_bytes);
-                    if (cr != CUDA_SUCCESS) return dev->fail(ANL_ERR_CUDA, "cuda: row_chain: shared memory limit");
-                }
-            }
             dev->chains[k2] = cp;
         }
         // slots share memory, and a caller may place an output over an input
@@ -701,6 +691,18 @@ int try_row_chain(anl_device* dev, const std::vector<Item>& items, size_t first,
             return pa == pb ? 1 : pa < pb + q.bytes && pb < pa + p.bytes ? 2 : 0;
         };
         if (cp && !chain_overwrites(members, reads, cp->r, place)) {
+            if (!cp->fn) {
+                std::shared_ptr<Module> mod;
+                if (int rc = compile_source(dev, cp->r.source, mod)) return rc;
+                CUfunction fn = nullptr;
+                CUresult cr = dev->drv.ModuleGetFunction(&fn, mod->mod, cp->r.entry.c_str());
+                if (cr != CUDA_SUCCESS) return dev->fail(ANL_ERR_CUDA, "cuda: row_chain entry point missing");
+                if (cp->r.smem_bytes) {
+                    cr = dev->drv.FuncSetAttribute(fn, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)cp->r.smem_bytes);
+                    if (cr != CUDA_SUCCESS) return dev->fail(ANL_ERR_CUDA, "cuda: row_chain: shared memory limit");
+                }
+                cp->fn = fn;
+            }
             std::vector<void*> ptrs;
             for (auto* m : members) for (auto& b : m->bufs) ptrs.push_back(t.bufs[b.id].ptr);
             std::vector<void*> args;
