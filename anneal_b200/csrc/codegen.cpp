@@ -2292,8 +2292,9 @@ bool render_row_chain(const std::vector<const Item*>& items, const std::vector<s
     k << "  (void)red_smem;\n" << aligned.str();
     std::string stages = decls + body.str();
     if (piped) {
-        // the next row is asked for once the first stage has used this one's registers: what the thread took from
-        // shared memory has arrived by then
+        // The next row is asked for after the first stage.  A thread copies into the place that it alone has read, and its
+        // reads come first in program order: those of operands that the first stage uses have arrived by then, the others
+        // rest on that order.
         k << "  { const int next = blockIdx.x;\n" << shift_decl("next") << fetch.str() << "  }\n";
         const size_t at = stages.find("@NEXT@");
         stages = stages.substr(0, at) + "if (row + (int)gridDim.x < " + std::to_string(rows) + ") { const int next = row + (int)gridDim.x;\n" + shift_decl("next") + fetch.str() + "  }\n" + stages.substr(at + 6);

@@ -48,7 +48,7 @@ struct Launch {
 
 struct Rendered {
     int klass = KC_ELEMENTWISE;
-    std::string source;            // one translation unit, may define two entry points
+    std::string source;            // one translation unit
     Launch main;
     // KC_REDUCE_SPLIT: blocks per output (-1: counted at launch from the bound batch, see split_parts), output
     // blocks (one ticket each), 32-bit partials one part writes, lanes per output, and for -1 the reduce

@@ -1,9 +1,7 @@
-// anl_sum_f32_static: the split scalar reduction (partials kernel + finish kernel) with its scratch
+// anl_sum_f32_static: a split scalar reduction (partials kernel + finish kernel) with its scratch
 // in a fixed device array instead of pool memory, for callers that must not reach the CUDA
-// allocator.  For n >= 65536 it mirrors, launch for launch, what the code generator emits for SUM
-// over one f32 buffer (the generator splits a reduction over several blocks from that length on;
-// shorter sums it runs in one block, so there the order of the additions differs from this file's
-// and the two agree to rounding, not bit for bit): every block reduces one contiguous chunk with 256
+// allocator.  It agrees to rounding with what the code generator emits for SUM over one f32 buffer (one launch
+// whose last block joins the parts), not bit for bit: here every block reduces one contiguous chunk with 256
 // lanes striding it, lanes are combined by an xor-shuffle butterfly and then across the eight warps
 // in ascending order, and one thread adds the partials in ascending order.  Nothing here allocates:
 // no cudaMalloc/cudaFree, no pool, no NVRTC.
@@ -79,7 +77,7 @@ extern "C" int anl_sum_f32_static(const float* x, int64_t n, float* out, void* s
         scratch = static_cast<float*>(p);
         g_scratch_addr[dev].store(scratch, std::memory_order_release);
     }
-    // same split the code generator picks for one output: about four blocks per SM, chunks of >= 4096
+    // about four blocks per SM, chunks of >= 4096
     long long parts = n / 4096;
     if (parts > 592) parts = 592;
     if (parts < 1) parts = 1;
