@@ -147,9 +147,11 @@ gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_con
 gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_constant__ TensorMap map_b, const SmallGemmArgs g) {
 #endif
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) unsigned long long full_bar[NSTAGE], empty_bar[NSTAGE], acc_full[CHUNK ? 2 : 1];
+    __shared__ __align__(8) unsigned long long full_bar[NSTAGE], empty_bar[NSTAGE];
 #if CFG_CHUNK
-    __shared__ __align__(8) unsigned long long acc_empty[2];
+    __shared__ __align__(8) unsigned long long acc_full[2], acc_empty[2];
+#else
+    __shared__ __align__(8) unsigned long long acc_full;
 #endif
     __shared__ unsigned tmem_base_slot;
     __shared__ volatile int failed;
@@ -166,10 +168,10 @@ gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_con
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < NSTAGE; s++) { mbar_init(smem_u32(&full_bar[s]), 1); mbar_init(smem_u32(&empty_bar[s]), 1); }
-        mbar_init(smem_u32(&acc_full[0]), 1);
 #if CFG_CHUNK
-        mbar_init(smem_u32(&acc_full[1]), 1);
-        for (int a = 0; a < 2; a++) mbar_init(smem_u32(&acc_empty[a]), 8);
+        for (int a = 0; a < 2; a++) { mbar_init(smem_u32(&acc_full[a]), 1); mbar_init(smem_u32(&acc_empty[a]), 8); }
+#else
+        mbar_init(smem_u32(&acc_full), 1);
 #endif
         failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -240,13 +242,13 @@ gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_con
             for (int ch = 0, first = 0; first < nkb && ok; ch++, first += CHUNK) {
             if (!mbar_wait(smem_u32(&acc_empty[ch & 1]), ((unsigned)(ch >> 1) & 1u) ^ 1u, &failed)) { ok = false; *(volatile int*)g.status = 24; break; }
             const int end = first + CHUNK < nkb ? first + CHUNK : nkb;
-#else
-            constexpr int ch = 0, first = 0;
-            const int end = nkb;
-            {
-#endif
             const unsigned acc = tmem_base + (ch & 1) * NT;
             for (int it = first; it < end; it++) {
+#else
+            constexpr int first = 0;
+            const unsigned acc = tmem_base;
+            for (int it = 0; it < nkb; it++) {
+#endif
                 if (!mbar_wait(smem_u32(&full_bar[stage]), phase, &failed)) { ok = false; *(volatile int*)g.status = 22; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const unsigned sp = smem_base + stage * STAGE_BYTES, sq = sp + P_BYTES;
@@ -256,7 +258,7 @@ gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_con
                 for (int pass = 0; pass < 3; pass++) {
                     const unsigned pp = pass == 0 ? sp + P_PART : sp, pq = pass == 1 ? sq + Q_PART : sq;
 #pragma unroll
-                    for (int k = 0; k < 4; k++) umma_f16(acc, make_desc(pp + k * 32, 16, 1024), make_desc(pq + k * 32, 16, 1024), idesc, it != first || (pass | k) != 0);
+                    for (int k = 0; k < 4; k++) umma_f16(acc, make_desc(pp + k * 32, 16, 1024), make_desc(pq + k * 32, 16, 1024), idesc, ((it - first) | pass | k) != 0);
                 }
 #else
 #pragma unroll
@@ -265,15 +267,20 @@ gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_con
                     // 128 bytes, 64-wide m/n groups one box apart.
                     const unsigned long long ad = CFG_A_MN ? make_desc(sp + k * 2048, BK * 128, 1024) : make_desc(sp + k * 32, 16, 1024);
                     const unsigned long long bd = CFG_B_MN ? make_desc(sq + k * 2048, BK * 128, 1024) : make_desc(sq + k * 32, 16, 1024);
-                    umma_f16(acc, ad, bd, idesc, it != first || k != 0);
+                    umma_f16(acc, ad, bd, idesc, ((it - first) | k) != 0);
                 }
 #endif
                 umma_commit(smem_u32(&empty_bar[stage]));
                 if (++stage == NSTAGE) { stage = 0; phase ^= 1; }
             }
+#if CFG_CHUNK
             if (ok) umma_commit(smem_u32(&acc_full[ch & 1]));
-            else failed = 1;
             }
+            if (!ok) failed = 1;
+#else
+            if (ok) umma_commit(smem_u32(&acc_full));
+            else failed = 1;
+#endif
         }
     }
     __syncwarp();
@@ -318,7 +325,7 @@ gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_con
     // ── every warp: its quadrant of the accumulator, half of the columns, to shared memory ──
     // The accumulator is complete, so every TMA write has been consumed and every MMA has read its operands: the
     // ring's memory is free.
-    bool ok = mbar_wait(smem_u32(&acc_full[0]), 0, &failed);
+    bool ok = mbar_wait(smem_u32(&acc_full), 0, &failed);
     if (!ok && lane == 0) { *(volatile int*)g.status = 23; failed = 1; }
     ok = __all_sync(0xffffffffu, ok);
     const int quad = warp & 3, half = warp >> 2;
