@@ -907,9 +907,19 @@ int run_items(anl_device* dev, const std::vector<Item>& items, const Bindings& b
             if (i + 1 < items.size() && N % 8 == 0 && !absorbed.count(i + 1)) {
                 fe = fused_epilogue_for(dev, it, items[i + 1], M, N);
                 if (fe->on) {
-                    // the consumer's output must not live in memory this contraction still reads
-                    void* o1 = t.bufs[items[i + 1].bufs[0].id].ptr;
-                    for (void* q : ptrs) if (q == o1) fe.reset();
+                    // The consumer's output must not live in memory this contraction still reads: the planner, for which the
+                    // contraction is over when its consumer starts, gives every second layer of a forward pass its input's
+                    // slot.  Such an output moves to a block of its own (a launch of 2.7 us and a round trip of the
+                    // activations saved, 32 x 4096 in f16); without one, and where it is not a slot, the two stay apart.
+                    DevBuf& o1 = t.bufs[items[i + 1].bufs[0].id];
+                    bool clash = false;
+                    for (void* q : ptrs) clash = clash || q == o1.ptr;
+                    void* own = nullptr;
+                    if (clash && items[i + 1].bufs[0].slot >= 0) {
+                        if (dev->alloc(o1.bytes, &own) == ANL_OK) { t.owned.push_back(own); o1.ptr = own; clash = false; }
+                        else cudaGetLastError();
+                    }
+                    if (clash) fe.reset();
                 }
                 if (fe && !fe->on) fe.reset();
             }
