@@ -70,6 +70,16 @@ constexpr int P_PART = CFG_PROWS * 128, Q_PART = NT * 128, P_BYTES = PARTS * P_P
 static_assert(!(CFG_TF32 && (CFG_A_MN || CFG_B_MN || CFG_EPI)), "the f32 form takes k-contiguous operands and no consumer");
 constexpr int LDT = NT + 4;              // floats per row of the staged f32 tile: rows 16 bytes apart in the banks
 constexpr int TMEM_COLS = CHUNK ? 2 * NT : NT;
+// Pieces of the finish (8 rows x 32 columns) that a warp takes together.  A piece alone is a chain of latencies (its operands
+// from L2, the arithmetic of an activation), and a warp has few of them to hide it behind: four at a time where registers hold
+// them and the partials are at hand, their operands asked for while the products are still running.  Training step of 1024 rows,
+// 4 x 1024 wide, 146.6 -> 143.3 us, of 999 rows 111.5 -> 109.9.  Where the partials come from other CTAs or chunks have taken
+// the registers, pieces by twos and fours were slower than one at a time (500 rows, 3 x 2048 wide, 67.8 us against 63.9).
+#if CFG_EPI
+constexpr int BATCH = SPLITS > 1 || CHUNK ? 1 : EPI_NRAW > 3 ? 2 : 4;
+#else
+constexpr int BATCH = SPLITS > 1 || CHUNK ? 1 : 4;
+#endif
 constexpr unsigned WAIT_LIMIT = 1u << 20;
 static_assert(!CFG_A_MN || CFG_PROWS == 128, "an m-contiguous operand is staged whole");
 static_assert(!CFG_B_MN || NT % 64 == 0, "an n-contiguous operand is staged in boxes of 64");
@@ -105,6 +115,12 @@ __device__ __forceinline__ float4 ld_cluster_f4(unsigned addr) {
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The same without an order on memory, where nothing that was written before is read after it and what was read has been
+// used: it does not wait for the stores of the outputs (32 rows through 4 x 4096, five launches, 60.4 -> 59.3 us).
+__device__ __forceinline__ void cluster_meet_all() {
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tma_load_2d(unsigned dst, const TensorMap* map, int c0, int c1, unsigned bar) {
     asm volatile(
@@ -285,6 +301,33 @@ gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_con
     }
     __syncwarp();
 
+    // pieces of the finish that this warp takes: piece j, its first row and column in the tile for this lane, and whether it has any
+    constexpr int WARPS = THREADS / 32;
+    const int per = g.colsum ? 4 : 1, units = (BM / 8 / per) * (NT / 32);
+    const int pieces = (units + SPLITS * WARPS - 1) / (SPLITS * WARPS) * per;
+    auto piece = [&](int j, int& trow, int& tcol) -> bool {
+        const int u = (int)rank * WARPS + warp + (per == 4 ? j >> 2 : j) * (SPLITS * WARPS);
+        const int rg = u / (NT / 32), cg = u - rg * (NT / 32);
+        trow = (rg * per + (per == 4 ? j & 3 : 0)) * 8 + (lane >> 2);
+        tcol = cg * 32 + 8 * (lane & 3);
+        return j < pieces && u < units && m0 + trow < g.M && n0 + tcol < g.N;
+    };
+#if CFG_EPI
+    // operands of BATCH pieces in registers: 16 of them for each operand
+    constexpr int EPI_NR = EPI_NRAW > 0 ? EPI_NRAW : 1;
+    __half2 raw[BATCH][EPI_NR][4];
+    auto load_operands = [&](int j0) {
+#pragma unroll
+        for (int q = 0; q < BATCH; q++) {
+            int trow, tcol;
+            if (piece(j0 + q, trow, tcol)) epi8_load_(m0 + trow, n0 + tcol, g.ep, raw[q]);
+        }
+    };
+#if !CFG_CHUNK
+    load_operands(0);
+#endif
+#endif
+
 #if CFG_CHUNK
     // ── the eight other warps: a quadrant of the accumulators each, half of the columns, from chunk to chunk in registers and
     // then to shared memory.  When the last chunk is complete, every TMA write has been consumed and every MMA has read
@@ -347,104 +390,111 @@ gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_con
     __syncthreads();
     if (SPLITS > 1) cluster_sync_all();                  // all partial tiles are in place
 
-    // ── sum of the partials, narrowing, fused consumer, stores: units of 8 rows x 32 columns, dealt out over all
-    // warps of the cluster (groups of four units when column sums over 32 rows are wanted).  Four lanes hold 64
+    // ── sum of the partials, narrowing, fused consumer, stores: pieces of 8 rows x 32 columns, dealt out over all
+    // warps of the cluster (four pieces below one another when column sums over 32 rows are wanted).  Four lanes hold 64
     // contiguous bytes of a row. ──
     const bool vec_ok = (g.N & 7) == 0;
-    const int per = g.colsum ? 4 : 1;
-    const int units = (BM / 8 / per) * (NT / 32);
 #if !CFG_TF32
     __half* const d_raw = (__half*)g.d_raw;
 #endif
     (void)vec_ok;
 #if CFG_EPI
     __half* const d_out = (__half*)g.d_out;
-    constexpr int EPI_NR = EPI_NRAW > 0 ? EPI_NRAW : 1;
 #endif
     if (!failed) {
-        for (int u = (int)rank * (THREADS / 32) + warp; u < units; u += SPLITS * (THREADS / 32)) {
-            const int rg = u / (NT / 32), cg = u - rg * (NT / 32);
-            const int tcol = cg * 32 + 8 * (lane & 3), col = n0 + tcol;
-            if (m0 + rg * 8 * per >= g.M || n0 + cg * 32 >= g.N) continue;      // warp-uniform
-            float x[8];
-#pragma unroll
-            for (int j = 0; j < 8; j++) x[j] = 0.0f;
-            for (int i = 0; i < per; i++) {
-                const int trow = (rg * per + i) * 8 + (lane >> 2), row = m0 + trow;
-                const bool on = row < g.M && col < g.N;
-                if (!on) continue;
-                float s[8];
+        float x[8];
+        for (int j0 = 0; j0 < pieces; j0 += BATCH) {
 #if CFG_EPI
-                __half2 raw[EPI_NR][4];
-                epi8_load_(row, col, g.ep, raw);
+            if (j0 > 0 || CHUNK) load_operands(j0);
 #endif
-                if (SPLITS == 1) {
-                    const float4 a = *reinterpret_cast<const float4*>(tile + trow * LDT + tcol), b = *reinterpret_cast<const float4*>(tile + trow * LDT + tcol + 4);
-                    s[0] = a.x; s[1] = a.y; s[2] = a.z; s[3] = a.w; s[4] = b.x; s[5] = b.y; s[6] = b.z; s[7] = b.w;
-                } else {
-                    const unsigned at = smem_u32(tile + trow * LDT + tcol);
-                    float4 a[SPLITS], b[SPLITS];
 #pragma unroll
-                    for (int r = 0; r < SPLITS; r++) { const unsigned p = map_to_cta(at, r); a[r] = ld_cluster_f4(p); b[r] = ld_cluster_f4(p + 16); }
+            {
+                constexpr int h = 0;
+                float4 a[BATCH][SPLITS], b[BATCH][SPLITS];
+                int trow[BATCH], tcol[BATCH];
+                bool on[BATCH];
 #pragma unroll
-                    for (int r = 0; r < SPLITS; r++) {
-                        if (r == 0) { s[0] = a[0].x; s[1] = a[0].y; s[2] = a[0].z; s[3] = a[0].w; s[4] = b[0].x; s[5] = b[0].y; s[6] = b[0].z; s[7] = b[0].w; }
-                        else { s[0] += a[r].x; s[1] += a[r].y; s[2] += a[r].z; s[3] += a[r].w; s[4] += b[r].x; s[5] += b[r].y; s[6] += b[r].z; s[7] += b[r].w; }
+                for (int q = 0; q < BATCH; q++) {
+                    on[q] = piece(j0 + h + q, trow[q], tcol[q]);
+                    if (!on[q]) continue;
+                    const float* const at = tile + trow[q] * LDT + tcol[q];
+                    if (SPLITS == 1) { a[q][0] = *reinterpret_cast<const float4*>(at); b[q][0] = *reinterpret_cast<const float4*>(at + 4); }
+                    else {
+#pragma unroll
+                        for (int r = 0; r < SPLITS; r++) { const unsigned p = map_to_cta(smem_u32(at), r); a[q][r] = ld_cluster_f4(p); b[q][r] = ld_cluster_f4(p + 16); }
                     }
                 }
-                const size_t off = (size_t)row * g.N + col;
+#pragma unroll
+                for (int q = 0; q < BATCH; q++) {
+                    const int j = j0 + h + q, row = m0 + trow[q], col = n0 + tcol[q];
+#if !CFG_TF32
+                    if ((j & 3) == 0) {
+#pragma unroll
+                        for (int e = 0; e < 8; e++) x[e] = 0.0f;
+                    }
+#endif
+                    if (on[q]) {
+                        float s[8] = {a[q][0].x, a[q][0].y, a[q][0].z, a[q][0].w, b[q][0].x, b[q][0].y, b[q][0].z, b[q][0].w};
+#pragma unroll
+                        for (int r = 1; r < SPLITS; r++) { s[0] += a[q][r].x; s[1] += a[q][r].y; s[2] += a[q][r].z; s[3] += a[q][r].w; s[4] += b[q][r].x; s[5] += b[q][r].y; s[6] += b[q][r].z; s[7] += b[q][r].w; }
+                        const size_t off = (size_t)row * g.N + col;
 #if CFG_TF32
-                float* const d = (float*)g.d_raw + off;
-                if ((g.N & 3) == 0) {
-                    *reinterpret_cast<float4*>(d) = make_float4(s[0], s[1], s[2], s[3]);
-                    if (col + 4 < g.N) *reinterpret_cast<float4*>(d + 4) = make_float4(s[4], s[5], s[6], s[7]);
-                } else {
+                        float* const d = (float*)g.d_raw + off;
+                        if ((g.N & 3) == 0) {
+                            *reinterpret_cast<float4*>(d) = make_float4(s[0], s[1], s[2], s[3]);
+                            if (col + 4 < g.N) *reinterpret_cast<float4*>(d + 4) = make_float4(s[4], s[5], s[6], s[7]);
+                        } else {
 #pragma unroll
-                    for (int j = 0; j < 8; j++) if (col + j < g.N) d[j] = s[j];
-                }
+                            for (int e = 0; e < 8; e++) if (col + e < g.N) d[e] = s[e];
+                        }
 #else
-                uint4 T;
-                __half2* const h = reinterpret_cast<__half2*>(&T);
+                        uint4 T;
+                        __half2* const t2 = reinterpret_cast<__half2*>(&T);
 #pragma unroll
-                for (int j = 0; j < 4; j++) h[j] = __floats2half2_rn(s[2 * j], s[2 * j + 1]);     // the single narrowing
-                if (vec_ok) {
-                    if (d_raw) *reinterpret_cast<uint4*>(d_raw + off) = T;
+                        for (int e = 0; e < 4; e++) t2[e] = __floats2half2_rn(s[2 * e], s[2 * e + 1]);     // the single narrowing
+                        if (vec_ok) {
+                            if (d_raw) *reinterpret_cast<uint4*>(d_raw + off) = T;
 #if CFG_EPI
-                    uint4 O;
-                    epi8_(row, col, h, reinterpret_cast<__half2*>(&O), g.ep, raw);
-                    *reinterpret_cast<uint4*>(d_out + off) = O;
-                    T = O;
+                            uint4 O;
+                            epi8_(row, col, t2, reinterpret_cast<__half2*>(&O), g.ep, raw[h + q]);
+                            *reinterpret_cast<uint4*>(d_out + off) = O;
+                            T = O;
 #endif
-                    if (g.colsum) {
+                            if (g.colsum) {
 #pragma unroll
-                        for (int j = 0; j < 4; j++) { const float2 f = __half22float2(h[j]); x[2 * j] += f.x; x[2 * j + 1] += f.y; }
-                    }
-                } else {
-                    // row stride not a multiple of 16 bytes (no fused consumer on this route)
+                                for (int e = 0; e < 4; e++) { const float2 f = __half22float2(t2[e]); x[2 * e] += f.x; x[2 * e + 1] += f.y; }
+                            }
+                        } else {
+                            // row stride not a multiple of 16 bytes (no fused consumer on this route)
 #pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        if (col + 2 * j < g.N) d_raw[off + 2 * j] = __low2half(h[j]);
-                        if (col + 2 * j + 1 < g.N) d_raw[off + 2 * j + 1] = __high2half(h[j]);
-                    }
-                }
+                            for (int e = 0; e < 4; e++) {
+                                if (col + 2 * e < g.N) d_raw[off + 2 * e] = __low2half(t2[e]);
+                                if (col + 2 * e + 1 < g.N) d_raw[off + 2 * e + 1] = __high2half(t2[e]);
+                            }
+                        }
 #endif
-            }
-            if (g.colsum) {
-                // the eight lanes of a column piece hold rows i * 8 + lane / 4: their sums, across the lanes
+                    }
+#if !CFG_TF32
+                    if (g.colsum && (j & 3) == 3) {
+                        // the eight lanes of a column piece hold rows i * 8 + lane / 4: their sums, across the lanes
 #pragma unroll
-                for (int o = 4; o <= 16; o <<= 1)
+                        for (int o = 4; o <= 16; o <<= 1)
 #pragma unroll
-                    for (int j = 0; j < 8; j++) x[j] += __shfl_xor_sync(0xffffffffu, x[j], o);
-                if (lane < 4 && col < g.N) {
-                    float* const cs = g.colsum + (size_t)((m0 >> 5) + rg) * g.N + col;
+                            for (int e = 0; e < 8; e++) x[e] += __shfl_xor_sync(0xffffffffu, x[e], o);
+                        const int row0 = m0 + (trow[q] & ~31);
+                        if (lane < 4 && j < pieces && row0 < g.M && col < g.N) {
+                            float* const cs = g.colsum + (size_t)(row0 >> 5) * g.N + col;
 #pragma unroll
-                    for (int j = 0; j < 8; j++) cs[j] = x[j];
+                            for (int e = 0; e < 8; e++) cs[e] = x[e];
+                        }
+                    }
+#endif
                 }
             }
         }
     }
     __syncthreads();
-    if (SPLITS > 1) cluster_sync_all();                  // the others' tiles stay until they have been read
+    if (SPLITS > 1) cluster_meet_all();                  // the others' tiles stay until they have been read
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
