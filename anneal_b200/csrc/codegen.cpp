@@ -498,6 +498,10 @@ struct Gen {
     std::string reduce_combine_mode;        // set by the kernel builder
     int lanes = 1, touts = 1, threads = 256; bool rc_layout = true;
 
+    // One reduce loop that serves several outputs (build_side_by_side): reduce_expr leaves its parts here instead of in `top`
+    struct SideBySide { bool on = false, ok = true; std::string tag, decl, head, body, acc; int reds = 0; } side;
+
+    std::vector<std::pair<Lin, int>>* loads_seen = nullptr;      // index and element size of every load rendered, while thread_order counts them
     Block prelude;                          // vector path: statements that must precede the unrolled loop
     Block* cur_top = nullptr;
     std::map<int, std::vector<bool>> atom_dep_memo;
@@ -819,6 +823,7 @@ struct Gen {
         int p = (int)N(nd.src[0]).arg;
         if (p < 0 || p >= (int)it.bufs.size()) { fail("codegen: PARAM number out of range"); return "0"; }
         Lin f = flat_index(i);
+        if (loads_seen) loads_seen->push_back({f, dt_storage_bytes(it.bufs[p].dtype)});
         auto cs = chain_subst.find(p);
         if (cs != chain_subst.end()) {
             // produced by an earlier stage of the same row chain: only this row's element is available
@@ -920,6 +925,22 @@ struct Gen {
         std::string acc = "acc" + std::to_string(i);
         std::vector<int> rr;
         for (size_t s = 1; s < nd.src.size(); s++) if (N(nd.src[s]).op == OP_RANGE) rr.push_back(nd.src[s]);
+        if (side.on) {
+            side.acc = acc + side.tag;
+            side.decl = std::string("  ") + at + " " + side.acc + " = " + identity(rop, acc_c) + ";\n";
+            const std::string e = val(nd.src[0], i), ef = (isf && cls(nd.src[0]) == CF16) ? "__half2float(" + e + ")" : e;
+            side.ok = side.ok && ++side.reds == 1 && !rr.empty() && T().code.empty();     // nothing may have been hoisted: the outputs share the text in front
+            std::string tot, vars, stride = "1";
+            for (int k = (int)rr.size() - 1; k >= 0; k--) {
+                const std::string rn = "r" + std::to_string(N(rr[k]).aux), b = range_bound(rr[k]);
+                vars += "    const int " + rn + " = " + (k == 0 ? "q / (" + stride + ")" : "(q / (" + stride + ")) % " + b) + "; (void)" + rn + ";\n";
+                stride += " * " + b;
+                tot = tot.empty() ? b : b + " * " + tot;
+            }
+            side.head = "  for (int q = RED_BEGIN(" + tot + "); q < RED_END(" + tot + "); q += RED_STEP) {\n" + vars;
+            side.body = "    {\n" + loop[i].code + "    " + side.acc + " = " + combine(rop, acc_c, side.acc, ef) + ";\n    }\n";
+            return nd.dtype == DT_F16 ? "__float2half_rn(" + side.acc + ")" : side.acc;
+        }
         stmt(-1, std::string(at) + " " + acc + " = " + identity(rop, acc_c) + ";");
         {
             if (enum_reduce.count(i) && lanes == 1 && rr.size() == 1) {
@@ -1657,15 +1678,17 @@ struct Gen {
         touts = threads / lanes;
     }
 
-    // `split`: parts per output, 0 = none, -1 = the kernel's nsplit argument.  `nob`: output blocks.
-    std::string reduce_macros(int split = 0, int64_t nob = 0) {
+    // `split`: parts per output, 0 = none, -1 = the kernel's nsplit argument.  `nob`: output blocks.  `wide`: elements a lane
+    // may take at once.
+    std::string reduce_macros(int split = 0, int64_t nob = 0, int wide = 8) {
         std::ostringstream m;
         m << "#define LANES " << lanes << "\n#define TOUTS " << touts << "\n#define RC_LAYOUT " << (rc_layout ? 1 : 0) << "\n";
         if (split) {
-            // each of an output's blocks owns a contiguous chunk of the flattened reduce space, a multiple of 8
+            // each of an output's blocks owns a contiguous chunk of the flattened reduce space, a multiple of `wide`
             // elements for every lane so that wide loads stay aligned
+            const std::string unit = "(" + std::to_string(wide) + " * LANES)";
             m << "#define SPLIT " << (split < 0 ? std::string("nsplit") : std::to_string(split)) << "\n#define NOB " << nob << "\n";
-            m << "#define RED_CHUNK(n) ((((n) + SPLIT - 1) / SPLIT + 8 * LANES - 1) / (8 * LANES) * (8 * LANES))\n";
+            m << "#define RED_CHUNK(n) ((((n) + SPLIT - 1) / SPLIT + " << unit << " - 1) / " << unit << " * " << unit << ")\n";
             m << "#define RED_LO(n) ((int)min((long long)part * RED_CHUNK(n), (long long)(n)))\n";
             m << "#define RED_BEGIN(n) (RED_LO(n) + lane)\n#define RED_BEGIN_V(n, v) (RED_LO(n) + lane * (v))\n";
             m << "#define RED_END(n) ((int)min((long long)(part + 1) * RED_CHUNK(n), (long long)(n)))\n#define RED_STEP LANES\n";
@@ -1832,6 +1855,157 @@ struct Gen {
         return true;
     }
 
+    // value of an affine form for given loop variables; `known` is cleared where it hangs on something else
+    int64_t lin_at(const Lin& l, const std::map<int, int64_t>& at, bool& known) const {
+        int64_t v = l.c;
+        for (auto& p : l.t) {
+            const Atom& a = atoms[p.first];
+            if (a.kind == Atom::RANGE) { auto f = at.find(a.node); v += p.second * (f == at.end() ? 0 : f->second); }
+            else if (a.kind == Atom::OPAQUE) known = false;
+            else { const int64_t x = lin_at(a.inner, at, known); v += p.second * (a.kind == Atom::DIV ? x / a.d : x % a.d); }
+        }
+        return v;
+    }
+    // 128-byte lines that a warp touches per output when neighbouring threads take neighbouring values of `order`'s last range:
+    // the loads `refs` and the store; averaged over a few warps.  < 0: not known.
+    double lines_touched(const std::vector<int>& order, const std::vector<std::pair<Lin, int>>& refs) {
+        const int64_t total = static_total();
+        double sum = 0;
+        const int64_t starts[4] = {0, total / 4 / 32 * 32, total / 2 / 32 * 32, total * 3 / 4 / 32 * 32};
+        for (int64_t g0 : starts) {
+            std::vector<std::set<int64_t>> seen(refs.size() + 1);
+            for (int64_t g = g0; g < g0 + 32 && g < total; g++) {
+                std::map<int, int64_t> at;
+                int64_t rem = g;
+                for (size_t k = order.size(); k-- > 0;) { at[order[k]] = rem % N(order[k]).arg; rem /= N(order[k]).arg; }
+                bool known = true;
+                for (size_t r = 0; r < refs.size(); r++) seen[r].insert(lin_at(refs[r].first, at, known) * refs[r].second >> 7);
+                int64_t o = 0;
+                for (int r : loop_ranges) o = o * N(r).arg + at[r];
+                seen.back().insert(o * dt_storage_bytes(it.bufs[0].dtype) >> 7);
+                if (!known) return -1;
+            }
+            for (auto& l : seen) sum += (double)l.size();
+        }
+        return sum / 4;
+    }
+    // Which range neighbouring threads should differ in when every thread works out one output by itself: the last one, unless
+    // another more than halves the lines touched.  A convolution with its channels last reads 16 channels' weights 288
+    // bytes apart in every warp; with the positions last they are one address and the image is contiguous: alone, 6 us of
+    // timing events included, 32 x 196 x 16 outputs of 72 taps 12.4 -> 9.2 us, 128 x 576 x 24 of 108 taps 197 -> 65.
+    std::vector<int> thread_order() {
+        std::vector<int> best = loop_ranges;
+        std::vector<std::pair<Lin, int>> refs;
+        loads_seen = &refs;
+        val(body, -1);
+        loads_seen = nullptr;
+        reset_emit();
+        const double as_is = lines_touched(loop_ranges, refs);
+        double least = as_is / 2;
+        if (as_is < 0) return best;
+        for (size_t k = 0; k + 1 < loop_ranges.size(); k++) {
+            if (N(loop_ranges[k]).arg < 16) continue;
+            std::vector<int> o = loop_ranges;
+            o.erase(o.begin() + k);
+            o.push_back(loop_ranges[k]);
+            const double c = lines_touched(o, refs);
+            if (c >= 0 && c < least) { least = c; best = o; }
+        }
+        return best;
+    }
+
+    // The enumerated outputs of a long reduction side by side: the innermost of the enumerated ranges (the 3 x 3 taps of a
+    // convolution's weight gradient) become accumulators of one thread, the others stay a switch.  As a block per output
+    // such a kernel reads the gradient once per tap and works out the same indexes (divisions by the image's extents, borders)
+    // for every term of every output, which is what bounded it.  Alone, 6 us of timing events included: 16 x 8 x 3 x 3
+    // outputs of 6272 terms 26.6 -> 11.3 us, 24 x 12 x 3 x 3 of 73728 218 -> 80, 8 x 1 x 3 x 3 of 25088 13.3 -> 10.2, 12 x 1 x 3 x 3 of
+    // 294912 53 -> 31.
+    bool build_side_by_side(Rendered& out, int64_t rmax, bool& taken) {
+        taken = false;
+        size_t nin = 0; int64_t ninner = 1;
+        while (nin < loop_ranges.size()) {
+            const int r = loop_ranges[loop_ranges.size() - 1 - nin];
+            if (std::find(enum_out.begin(), enum_out.end(), r) == enum_out.end() || ninner * N(r).arg > 16) break;
+            ninner *= N(r).arg; nin++;
+        }
+        if (nin == 0 || ninner < 4 || rmax < 1024) return true;
+        const std::vector<int> inner(loop_ranges.end() - nin, loop_ranges.end());
+        std::vector<int> outer;
+        for (int r : enum_out) if (std::find(inner.begin(), inner.end(), r) == inner.end()) outer.push_back(r);
+        auto fix_all = [&](const std::vector<int>& rs, int64_t v) { for (size_t e = rs.size(); e-- > 0;) { fix_range(rs[e], v % N(rs[e]).arg); v /= N(rs[e]).arg; } };
+        int64_t cases = 1;
+        for (int r : outer) cases *= N(r).arg;
+        // blocks of up to 1024 lanes an output group; with few groups, parts of four trips a lane or more in several blocks
+        const int64_t groups = static_total() / ninner;
+        int L = 256, parts = 1;
+        if (groups >= 74) { while (L < 1024 && groups * L < 148 * 1024 && rmax / (L * 2) >= 4) L *= 2; }
+        else parts = (int)std::max<int64_t>(1, std::min<int64_t>({(rmax + L * 4 - 1) / (L * 4), 148 * 2 / groups, 1024}));
+        if (groups > kMaxTickets && parts > 1) parts = 1;
+        rc_layout = true; lanes = threads = L; touts = 1;
+
+        const int red = reduces[0], rop = (int)N(red).aux;
+        const Cls c0 = dtype_cls(N(red).dtype);
+        const bool isf = c0 == CF32 || c0 == CF16;
+        const Cls acc_c = isf ? CF32 : c0;
+        const std::string tag = std::string(rop_tag(rop)) + "_" + (isf ? "f" : "i"), at = isf ? "float" : cls_ctype(acc_c);
+        reset_emit();
+        reduce_combine_mode.clear();
+        std::string text;
+        for (int64_t cs = 0; cs < cases && side.ok; cs++) {
+            fix_all(outer, cs);
+            std::string decl, head, body_text, group, finish;
+            for (int64_t in = 0; in < ninner && side.ok; in++) {
+                fix_all(inner, in);
+                top = Block(); loop.clear(); memo.clear();
+                side = SideBySide(); side.on = true; side.tag = "_" + std::to_string(in);
+                const std::string v = val(body, -1);
+                if (!err.empty() || side.reds != 1) side.ok = false;
+                const std::string num = std::to_string(in);
+                decl += side.decl; head = side.head; body_text += side.body;
+                group += "  _Pragma(\"unroll\") for (int o = 16; o > 0; o >>= 1) " + side.acc + " = op_" + tag + "(" + side.acc + ", __shfl_xor_sync(0xffffffffu, " + side.acc + ", o));\n" +
+                         "  if ((threadIdx.x & 31) == 0) sums[" + num + " * (LANES / 32) + (threadIdx.x >> 5)] = " + side.acc + ";\n";
+                finish += "  if (lane == " + num + ") {\n  const " + at + " " + side.acc + " = mine;\n" + top.code + "  data0[g * " + std::to_string(ninner) + " + " + num + "] = " + store_value(v, body) + ";\n  }\n";
+            }
+            // the warps' sums together, added in order by one thread an output
+            text += "  case " + std::to_string(cs) + ": {\n" + decl + head + body_text + "  }\n" + group + "  __syncthreads();\n";
+            text += "  " + at + " mine = " + identity(rop, acc_c) + ";\n  if (lane < " + std::to_string(ninner) + ") { mine = sums[lane * (LANES / 32)]; for (int w = 1; w < LANES / 32; w++) mine = op_" + tag + "(mine, sums[lane * (LANES / 32) + w]); }\n";
+            if (parts > 1) {
+                const std::string cell = "NOB + ob) * " + std::to_string(ninner) + " + lane";
+                text += "  " + at + "* const sc = reinterpret_cast<" + at + "*>(scratch);\n  if (lane < " + std::to_string(ninner) + ") { sc[((long long)part * " + cell + "] = mine; __threadfence(); }\n  __syncthreads();\n";
+                text += "  if (threadIdx.x == 0) { split_last = atomicAdd(tickets + ob, 1u) == (unsigned)SPLIT - 1u; if (split_last) tickets[ob] = 0u; }\n";
+                text += "  __syncthreads();\n  if (!split_last) return;\n  __threadfence();\n";
+                text += "  if (lane < " + std::to_string(ninner) + ") { mine = " + identity(rop, acc_c) + "; _Pragma(\"unroll 8\") for (int p = 0; p < SPLIT; p++) mine = op_" + tag + "(mine, __ldcg(sc + ((long long)p * " + cell + ")); }\n";
+            }
+            text += finish + "  } break;\n";
+        }
+        for (int r : enum_out) unfix_range(r);
+        const bool ok = side.ok && err.empty();
+        side = SideBySide();
+        if (!ok) return err.empty();
+        std::ostringstream k;
+        k << reduce_macros(parts > 1 ? parts : 0, groups, 1) << preamble();
+        k << signature("reduce_fused", parts > 1, threads) << " {\n  enter_();\n";
+        k << "  __shared__ " << at << " sums[" << ninner * (threads / 32) << "];\n  const int lane = threadIdx.x;\n";
+        if (parts > 1) k << "  __shared__ unsigned split_last;\n  const int ob = blockIdx.x / SPLIT, part = blockIdx.x % SPLIT;\n  const long long g = ob;\n";
+        else k << "  const long long g = blockIdx.x;\n";
+        k << decompose("g", 0, loop_ranges.size() - nin);
+        std::string sel = "0";
+        for (int r : outer) sel = "(" + sel + " * " + std::to_string(N(r).arg) + " + r" + std::to_string(N(r).aux) + ")";
+        k << "  switch (" << sel << ") {\n" << text << "  }\n}\n";
+        out.klass = parts > 1 ? KC_REDUCE_SPLIT : KC_REDUCE;
+        out.source = k.str();
+        out.main.entry = "reduce_fused";
+        out.main.block = threads;
+        out.main.outputs_per_block = 1;
+        out.main.static_outputs = groups;
+        if (parts > 1) { out.split = parts; out.out_blocks = groups; out.part_elems = groups * ninner; out.split_lanes = lanes; }
+        out.note = "reduce RC lanes=" + std::to_string(lanes) + " " + std::to_string(ninner) + " outputs side by side";
+        if (parts > 1) out.note += " split reduce parts=" + std::to_string(parts);
+        if (!outer.empty()) out.note += " switch over " + std::to_string(outer.size()) + " output ranges";
+        taken = true;
+        return true;
+    }
+
     bool build_reduce(Rendered& out) {
         if (opts.reduce_lanes == 0 && opts.split <= 1 && !opts.sym_split && enum_out.empty() && enum_reduce.empty()) {
             size_t ninv = 0; int64_t inner = 1;
@@ -1848,6 +2022,11 @@ struct Gen {
         int64_t total = static_total();
         int64_t rmax = 0; bool rsym = false;
         for (int r : reduces) { int64_t t = reduce_total(r); if (t == 0) rsym = true; rmax = std::max(rmax, t); }
+        if (!enum_out.empty() && enum_reduce.empty() && reduces.size() == 1 && !rsym && !sym_output() && opts.split <= 1 && opts.reduce_lanes == 0 && opts.block_threads == 0) {
+            bool taken = false;
+            if (!build_side_by_side(out, rmax, taken)) return false;
+            if (taken) return true;
+        }
         const bool dyn = opts.sym_split;         // the form of a REDUCE over the bound batch whose parts are counted at launch
         if (dyn && !(rsym && reduces.size() == 1 && !sym_output())) return fail("codegen: no split over the bound batch");
         if (rsym) rmax = dyn ? (int64_t)1 << 20 : 0;
@@ -1915,12 +2094,24 @@ struct Gen {
         } else k << "  long long g = (long long)blockIdx.x * TOUTS + grp;\n";
         k << "  const bool valid = g < " << total_expr() << ";\n";
         k << "  if (!valid) g = " << total_expr() << " - 1;\n";
-        k << decompose("g");
+        std::string at = "g";
+        if (!enum_reduce.empty() && lanes == 1 && !split_mode && !has_sym) {
+            const std::vector<int> order = thread_order(), natural = loop_ranges;
+            if (order != natural) {
+                loop_ranges = order;
+                k << decompose("g");
+                loop_ranges = natural;
+                at = "";
+                int64_t stride = 1;
+                for (size_t r = natural.size(); r-- > 0;) { at += (at.empty() ? "r" : " + r") + std::to_string(N(natural[r]).aux) + " * " + std::to_string(stride) + "LL"; stride *= N(natural[r]).arg; }
+            }
+        }
+        if (at == "g") k << decompose("g");
         if (enum_out.empty()) {
             std::string v = val(body, -1);
             if (!err.empty()) return false;
             k << top.code;
-            k << "  if (valid && lane == 0) data0[g] = " << store_value(v, body) << ";\n";
+            k << "  if (valid && lane == 0) data0[" << at << "] = " << store_value(v, body) << ";\n";
         } else {
             if (!emit_cases(k, "  if (valid && lane == 0) data0[g] = ")) return false;
         }
