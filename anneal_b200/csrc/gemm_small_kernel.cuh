@@ -482,7 +482,7 @@ gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_con
 #pragma unroll
                             for (int e = 0; e < 8; e++) x[e] += __shfl_xor_sync(0xffffffffu, x[e], o);
                         const int row0 = m0 + (trow[q] & ~31);
-                        if (lane < 4 && j < pieces && row0 < g.M && col < g.N) {
+                        if (lane < 4 && trow[q] < BM && row0 < g.M && col < g.N) {        // warps past the last unit have rows past the tile
                             float* const cs = g.colsum + (size_t)(row0 >> 5) * g.N + col;
 #pragma unroll
                             for (int e = 0; e < 8; e++) cs[e] = x[e];
