@@ -359,23 +359,43 @@ SmallVariant choose_small(const GemmPlan& gp, int64_t M) {
     return v;
 }
 
-std::string small_source(const SmallVariant& v, const std::string& epilogue) {
+// `name`: empty for a kernel of its own, else the namespace of one of two configurations in a text
+std::string small_source(const SmallVariant& v, const std::string& epilogue, const std::string& name = std::string()) {
     std::string s;
     s += "#define ANL_SMALL_GEMM_DEVICE_CODE 1\n";
+    s += "#define CFG_NAME " + (name.empty() ? std::string("alone") : name) + "\n#define CFG_ALONE " + (name.empty() ? "1" : "0") + "\n";
     s += "#define CFG_A_MN " + std::to_string(v.a_mn ? 1 : 0) + "\n#define CFG_B_MN " + std::to_string(v.b_mn ? 1 : 0) + "\n";
     s += "#define CFG_NT " + std::to_string(v.nt) + "\n#define CFG_PROWS " + std::to_string(v.prows) + "\n";
     s += "#define CFG_STAGES " + std::to_string(v.stages) + "\n#define CFG_SPLITS " + std::to_string(v.splits) + "\n";
     s += "#define CFG_EPI " + std::string(epilogue.empty() ? "0" : "1") + "\n";
     s += "#define CFG_TF32 " + std::string(v.tf32 ? "1" : "0") + "\n#define CFG_CHUNK " + std::to_string(v.chunk) + "\n";
-    s += epilogue;
+    if (name.empty()) s += epilogue;
+    else if (!epilogue.empty()) s += "#include <cuda_fp16.h>\nnamespace " + name + " {\n" + epilogue + "}\n";
     s += kSmallKernelSource;
     return s;
 }
 
-int get_small_kernel(anl_device* dev, const SmallVariant& v, const std::string& epilogue, CUfunction* fn) {
+// Both configurations in one kernel: the first `ctas` CTAs are the first one's.
+std::string small_pair_source(const SmallVariant& v0, const std::string& epi0, const SmallVariant& v1, const std::string& epi1) {
+    std::string s = small_source(v0, epi0, "first");
+    for (const char* m : {"ANL_SMALL_GEMM_DEVICE_CODE", "CFG_NAME", "CFG_ALONE", "CFG_A_MN", "CFG_B_MN", "CFG_NT", "CFG_PROWS", "CFG_STAGES", "CFG_SPLITS", "CFG_EPI", "CFG_TF32", "CFG_CHUNK", "EPI_NRAW"}) s += std::string("#undef ") + m + "\n";
+    s += small_source(v1, epi1, "second");
+    s += "extern \"C\" __global__ void __launch_bounds__(first::THREADS, 2)\n"
+         "gemm_f16_tcgen05_small_two(const __grid_constant__ TensorMap map_a0, const __grid_constant__ TensorMap map_b0, const __grid_constant__ TensorMap map_a1,\n"
+         "                           const __grid_constant__ TensorMap map_b1, const __grid_constant__ SmallGemmArgs g0, const __grid_constant__ SmallGemmArgs g1, const unsigned ctas) {\n"
+         "    static_assert(first::THREADS == second::THREADS && first::SPLITS == second::SPLITS, \"one launch, one block and cluster shape\");\n"
+         "    if (blockIdx.x < ctas) first::run(map_a0, map_b0, g0, blockIdx.x);\n"
+         "    else second::run(map_a1, map_b1, g1, blockIdx.x - ctas);\n}\n";
+    return s;
+}
+
+std::string small_key(const SmallVariant& v, const std::string& epilogue) {
     char head[96];
     std::snprintf(head, sizeof head, "s%d,%d,%d,%d,%d,%d,%d,%d|", v.nt, v.prows, v.stages, v.splits, v.chunk, (int)v.a_mn, (int)v.b_mn, (int)v.tf32);
-    const std::string key = head + epilogue;
+    return head + epilogue;
+}
+int get_small_kernel(anl_device* dev, const SmallVariant& v, const std::string& epilogue, CUfunction* fn) {
+    const std::string key = small_key(v, epilogue);
     auto hit = dev->pair_kernels.find(key);
     if (hit != dev->pair_kernels.end()) { *fn = (CUfunction)hit->second; return ANL_OK; }
     return load_gemm_kernel(dev, small_source(v, epilogue), "gemm_f16_tcgen05_small", small_smem_bytes(v), key, fn);
@@ -396,6 +416,36 @@ bool small_takes(const GemmPlan& gp, int64_t M) {
 }
 
 }  // namespace
+
+// A one-CTA launch that is ready but waits for the next contraction.
+struct HeldGemm { SmallVariant v; std::string epilogue; CUtensorMap ma, mb; SmallGemmArgs g; int64_t ctas; };
+void drop_held(HeldGemm* h) { delete h; }
+bool gemm_holdable(const Plan& plan) { return gemm_fusable(plan) && !plan.gemm->pad_a && !plan.gemm->pad_b && small_takes(*plan.gemm, plan.gemm->c.M); }
+// One CTA of each on an SM, and one launch's shape for both.  (The larger ones fill the machine by themselves.)
+bool gemm_pairs(const HeldGemm& a, const HeldGemm& b) {
+    return a.v.splits == b.v.splits && a.v.threads() == b.v.threads() && a.ctas <= 148 && b.ctas <= 148 &&
+           small_smem_bytes(a.v) <= 110 * 1024 && small_smem_bytes(b.v) <= 110 * 1024;
+}
+int launch_held(anl_device* dev, HeldGemm& a, HeldGemm* b, cudaStream_t stream) {
+    CUfunction fn;
+    if (!b) {
+        if (int rc = get_small_kernel(dev, a.v, a.epilogue, &fn)) return rc;
+        void* params[3] = {&a.ma, &a.mb, &a.g};
+        if (int rc = launch_kernel(dev, fn, KernelShape{(unsigned)a.ctas, 1, 1, (unsigned)a.v.threads(), 1, 1, (unsigned)small_smem_bytes(a.v), (unsigned)a.v.splits}, stream, params, true, "gemm_f16_tcgen05_small")) return rc;
+        dev->stats.gemm_launched++;
+        return ANL_OK;
+    }
+    const int smem = std::max(small_smem_bytes(a.v), small_smem_bytes(b->v));
+    const std::string key = small_key(a.v, a.epilogue) + "&" + small_key(b->v, b->epilogue);
+    auto hit = dev->pair_kernels.find(key);
+    if (hit != dev->pair_kernels.end()) fn = (CUfunction)hit->second;
+    else if (int rc = load_gemm_kernel(dev, small_pair_source(a.v, a.epilogue, b->v, b->epilogue), "gemm_f16_tcgen05_small_two", smem, key, &fn)) return rc;
+    unsigned ctas = (unsigned)a.ctas;
+    void* params[7] = {&a.ma, &a.mb, &b->ma, &b->mb, &a.g, &b->g, &ctas};
+    if (int rc = launch_kernel(dev, fn, KernelShape{(unsigned)(a.ctas + b->ctas), 1, 1, (unsigned)a.v.threads(), 1, 1, (unsigned)smem, (unsigned)a.v.splits}, stream, params, true, "gemm_f16_tcgen05_small_two")) return rc;
+    dev->stats.gemm_launched += 2;
+    return ANL_OK;
+}
 
 int gemm_small_parts(const Plan& plan) {
     if (!gemm_fusable(plan) || !small_takes(*plan.gemm, plan.gemm->c.M)) return 0;
@@ -653,7 +703,7 @@ static int launch_gemm_tf32x3(anl_device* dev, const GemmPlan& gp, const float* 
 }
 
 int launch_gemm(anl_device* dev, const Plan& plan, void* const* bufs, int64_t sym_value, cudaStream_t stream, int64_t m_begin, int64_t m_end,
-                const GemmFusion* fusion, std::vector<void*>* keep_scratch, bool b_settled) {
+                const GemmFusion* fusion, std::vector<void*>* keep_scratch, bool b_settled, HeldGemm** hold) {
     const GemmPlan& gp = *plan.gemm;
     const Contraction& c = gp.c;
     // an optional row window [m_begin, m_end) of the output: the caller splits a contraction so that
@@ -708,8 +758,6 @@ int launch_gemm(anl_device* dev, const Plan& plan, void* const* bufs, int64_t sy
         if (gp.b_mn) rc = encode_map(dev, &mb, b, (uint64_t)c.N, (uint64_t)c.K, (uint64_t)ldb, 64, BK);
         else rc = encode_map(dev, &mb, b, (uint64_t)c.K, (uint64_t)c.N, (uint64_t)ldb, BK, v.nt);
         if (rc) return done(rc);
-        CUfunction fn;
-        if ((rc = get_small_kernel(dev, v, fusion && fusion->epilogue ? *fusion->epilogue : std::string(), &fn))) return done(rc);
         SmallGemmArgs g{};
         __half* out0 = (__half*)bufs[0] + (window ? m_begin * c.N : 0);
         g.d_raw = (!fusion || fusion->store_raw) ? out0 : nullptr;
@@ -722,9 +770,9 @@ int launch_gemm(anl_device* dev, const Plan& plan, void* const* bufs, int64_t sy
         const int64_t ctas = (int64_t)g.tiles_m * ((c.N + v.nt - 1) / v.nt) * v.splits;
         if (ctas > 0x7fffffffLL) return done(dev->fail(ANL_ERR_LIMIT, "gemm: grid too large"));
         g.b_settled = b_settled && !gp.pad_b;
-        void* params[3] = {&ma, &mb, &g};
-        if ((rc = launch_kernel(dev, fn, KernelShape{(unsigned)ctas, 1, 1, (unsigned)v.threads(), 1, 1, (unsigned)small_smem_bytes(v), (unsigned)v.splits}, stream, params, true, "gemm_f16_tcgen05_small"))) return done(rc);
-        dev->stats.gemm_launched++;
+        HeldGemm h{v, fusion && fusion->epilogue ? *fusion->epilogue : std::string(), ma, mb, g, ctas};
+        if (hold && !window && !gp.pad_a && !gp.pad_b) { *hold = new HeldGemm(std::move(h)); return ANL_OK; }
+        if ((rc = launch_held(dev, h, nullptr, stream))) return done(rc);
         return done(ANL_OK);
     }
     if (gp.a_mn) rc = encode_map(dev, &ma, a, (uint64_t)M, (uint64_t)c.K, (uint64_t)lda, 64, BK);

@@ -45,7 +45,15 @@
 //   CFG_CHUNK            k-blocks accumulated in tensor memory at a time; 0 when no slice is longer than a chunk
 //   CFG_TF32             1: f32 operands as hi and lo parts, f32 output (k-contiguous only, no fused consumer, no column sums)
 //   CFG_EPI              1 when a fused elementwise consumer has been prepended (gemm_pair_kernel.cuh says how)
-#pragma once
+//   CFG_NAME             namespace of this configuration
+//   CFG_ALONE            1: the text ends in a kernel of its own; 0: it is there twice, and the host appends the kernel of both
+//
+// Two contractions that do not depend on each other, a layer's weight gradient and its input gradient, run as ONE launch of
+// both configurations: one CTA of each sits on an SM, so that one's loads (94 bytes a ns for a ring of 100 KB, of the 145 an
+// SM can take from L2) and finish run beside the other's, and one launch's fixed cost is saved.  Training step of 1024 rows,
+// 4 x 1024 wide, 144.1 -> 130.4 us, of 999 rows, 2 x 1000 wide, 111.0 -> 97.2.
+#ifndef ANL_SMALL_GEMM_COMMON
+#define ANL_SMALL_GEMM_COMMON
 
 struct SmallGemmArgs {
     void* d_raw;            // [M, N] f16 (f32): the contraction itself; null when nothing else reads it
@@ -64,25 +72,7 @@ struct SmallGemmArgs {
 
 struct alignas(64) TensorMap { unsigned long long opaque[16]; };
 
-// a k-block is one 128-byte swizzle row of k: 64 f16 or 32 f32 elements; in the f32 form each operand is staged as hi, then lo
-constexpr int BM = 128, BK = CFG_TF32 ? 32 : 64, PARTS = CFG_TF32 ? 2 : 1, NT = CFG_NT, NSTAGE = CFG_STAGES, SPLITS = CFG_SPLITS, CHUNK = CFG_CHUNK, THREADS = CHUNK ? 320 : 256;
-constexpr int P_PART = CFG_PROWS * 128, Q_PART = NT * 128, P_BYTES = PARTS * P_PART, STAGE_BYTES = P_BYTES + PARTS * Q_PART;
-static_assert(!(CFG_TF32 && (CFG_A_MN || CFG_B_MN || CFG_EPI)), "the f32 form takes k-contiguous operands and no consumer");
-constexpr int LDT = NT + 4;              // floats per row of the staged f32 tile: rows 16 bytes apart in the banks
-constexpr int TMEM_COLS = CHUNK ? 2 * NT : NT;
-// Pieces of the finish (8 rows x 32 columns) that a warp takes together.  A piece alone is a chain of latencies (its operands
-// from L2, the arithmetic of an activation), and a warp has few of them to hide it behind: four at a time where registers hold
-// them and the partials are at hand, their operands asked for while the products are still running.  Training step of 1024 rows,
-// 4 x 1024 wide, 146.6 -> 143.3 us, of 999 rows 111.5 -> 109.9.  Where the partials come from other CTAs or chunks have taken
-// the registers, pieces by twos and fours were slower than one at a time (500 rows, 3 x 2048 wide, 67.8 us against 63.9).
-#if CFG_EPI
-constexpr int BATCH = SPLITS > 1 || CHUNK ? 1 : EPI_NRAW > 3 ? 2 : 4;
-#else
-constexpr int BATCH = SPLITS > 1 || CHUNK ? 1 : 4;
-#endif
 constexpr unsigned WAIT_LIMIT = 1u << 20;
-static_assert(!CFG_A_MN || CFG_PROWS == 128, "an m-contiguous operand is staged whole");
-static_assert(!CFG_B_MN || NT % 64 == 0, "an n-contiguous operand is staged in boxes of 64");
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count)); }
@@ -133,16 +123,6 @@ __device__ __forceinline__ unsigned long long make_desc(unsigned saddr, unsigned
     return (unsigned long long)((saddr >> 4) & 0x3FFF) | ((unsigned long long)((lbo_bytes >> 4) & 0x3FFF) << 16) |
            ((unsigned long long)((sbo_bytes >> 4) & 0x3FFF) << 32) | (1ull << 46) | (2ull << 61);
 }
-__device__ __forceinline__ void umma_f16(unsigned tmem_d, unsigned long long adesc, unsigned long long bdesc, unsigned idesc, unsigned accumulate) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-#if CFG_TF32
-        " tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}\n"
-#else
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-#endif
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
 __device__ __forceinline__ void umma_commit(unsigned bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -155,13 +135,49 @@ __device__ __forceinline__ void tmem_ld16(unsigned taddr, unsigned* v) {
         : "r"(taddr) : "memory");
 }
 
-extern "C" __global__ void __launch_bounds__(THREADS, 2)
-#if CFG_TF32
-gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_constant__ TensorMap map_b,
-                       const __grid_constant__ TensorMap map_a_lo, const __grid_constant__ TensorMap map_b_lo, const SmallGemmArgs g) {
+#endif  // ANL_SMALL_GEMM_DEVICE_CODE
+#endif  // ANL_SMALL_GEMM_COMMON
+
+#ifdef ANL_SMALL_GEMM_DEVICE_CODE
+namespace CFG_NAME {
+
+// a k-block is one 128-byte swizzle row of k: 64 f16 or 32 f32 elements; in the f32 form each operand is staged as hi, then lo
+constexpr int BM = 128, BK = CFG_TF32 ? 32 : 64, PARTS = CFG_TF32 ? 2 : 1, NT = CFG_NT, NSTAGE = CFG_STAGES, SPLITS = CFG_SPLITS, CHUNK = CFG_CHUNK, THREADS = CHUNK ? 320 : 256;
+constexpr int P_PART = CFG_PROWS * 128, Q_PART = NT * 128, P_BYTES = PARTS * P_PART, STAGE_BYTES = P_BYTES + PARTS * Q_PART;
+static_assert(!(CFG_TF32 && (CFG_A_MN || CFG_B_MN || CFG_EPI)), "the f32 form takes k-contiguous operands and no consumer");
+constexpr int LDT = NT + 4;              // floats per row of the staged f32 tile: rows 16 bytes apart in the banks
+constexpr int TMEM_COLS = CHUNK ? 2 * NT : NT;
+// Pieces of the finish (8 rows x 32 columns) that a warp takes together.  A piece alone is a chain of latencies (its operands
+// from L2, the arithmetic of an activation), and a warp has few of them to hide it behind: four at a time where registers hold
+// them and the partials are at hand, their operands asked for while the products are still running.  Training step of 1024 rows,
+// 4 x 1024 wide, 146.6 -> 143.3 us, of 999 rows 111.5 -> 109.9.  Where the partials come from other CTAs or chunks have taken
+// the registers, pieces by twos and fours were slower than one at a time (500 rows, 3 x 2048 wide, 67.8 us against 63.9).
+#if CFG_EPI
+constexpr int BATCH = SPLITS > 1 || CHUNK ? 1 : EPI_NRAW > 3 ? 2 : 4;
 #else
-gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_constant__ TensorMap map_b, const SmallGemmArgs g) {
+constexpr int BATCH = SPLITS > 1 || CHUNK ? 1 : 4;
 #endif
+static_assert(!CFG_A_MN || CFG_PROWS == 128, "an m-contiguous operand is staged whole");
+static_assert(!CFG_B_MN || NT % 64 == 0, "an n-contiguous operand is staged in boxes of 64");
+
+
+__device__ __forceinline__ void umma_f16(unsigned tmem_d, unsigned long long adesc, unsigned long long bdesc, unsigned idesc, unsigned accumulate) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+#if CFG_TF32
+        " tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}\n"
+#else
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+#endif
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+
+// `block`: number of this CTA among the contraction's own
+__device__ __forceinline__ void run(const TensorMap& map_a, const TensorMap& map_b,
+#if CFG_TF32
+                                    const TensorMap& map_a_lo, const TensorMap& map_b_lo,
+#endif
+                                    const SmallGemmArgs& g, const unsigned block) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) unsigned long long full_bar[NSTAGE], empty_bar[NSTAGE];
 #if CFG_CHUNK
@@ -176,7 +192,7 @@ gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_con
     float* const tile = reinterpret_cast<float*>(smem_raw + (smem_base - smem_u32(smem_raw)));   // the ring's memory, once the ring is done
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned rank = SPLITS > 1 ? cluster_ctarank() : 0u;
-    const int t = (int)(blockIdx.x / SPLITS);
+    const int t = (int)(block / SPLITS);
     const int m0 = (t % g.tiles_m) * BM, n0 = (t / g.tiles_m) * NT;
     const int kblocks = (g.K + BK - 1) / BK;
     // this CTA's slice: at least one k-block, as the host gives no tile more CTAs than it has k-blocks
@@ -501,4 +517,20 @@ gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_con
     }
 }
 
+}  // namespace CFG_NAME
+
+#if CFG_ALONE
+#if CFG_TF32
+extern "C" __global__ void __launch_bounds__(CFG_NAME::THREADS, 2)
+gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_constant__ TensorMap map_b,
+                       const __grid_constant__ TensorMap map_a_lo, const __grid_constant__ TensorMap map_b_lo, const __grid_constant__ SmallGemmArgs g) {
+    CFG_NAME::run(map_a, map_b, map_a_lo, map_b_lo, g, blockIdx.x);
+}
+#else
+extern "C" __global__ void __launch_bounds__(CFG_NAME::THREADS, 2)
+gemm_f16_tcgen05_small(const __grid_constant__ TensorMap map_a, const __grid_constant__ TensorMap map_b, const __grid_constant__ SmallGemmArgs g) {
+    CFG_NAME::run(map_a, map_b, g, blockIdx.x);
+}
+#endif
+#endif
 #endif  // ANL_SMALL_GEMM_DEVICE_CODE

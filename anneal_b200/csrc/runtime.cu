@@ -848,9 +848,55 @@ int run_items(anl_device* dev, const std::vector<Item>& items, const Bindings& b
     std::set<const void*> written;
     if (keep_scratch) for (auto& it : items) written.insert(t.bufs[it.bufs[0].id].ptr);
     auto settled = [&](const Plan& p, const std::vector<void*>& ptrs) { return keep_scratch && gemm_fusable(p) && !written.count(ptrs[gemm_b_param(p)]); };
+    // Two contractions in a row that do not depend on each other (a layer's weight gradient, then the gradient of its input)
+    // are one launch where both are small (gemm_small_kernel.cuh): the first waits here, prepared, until the second is.
+    // Only when the very next item is such a contraction, so that nothing is launched between them.
+    struct Span { const char* at; size_t bytes; };
+    struct Pending { std::unique_ptr<HeldGemm, void (*)(HeldGemm*)> held{nullptr, drop_held}; std::vector<Span> reads, writes; std::function<int()> after; size_t item = 0; } pending;
+    const bool pairs_on = dev->nranks <= 1 && !dev->profiling && !(dev->flags & ANL_OPEN_BEAM);
+    auto meet = [](const std::vector<Span>& a, const std::vector<Span>& b) {
+        for (const Span& x : a) for (const Span& y : b) if (x.at < y.at + y.bytes && y.at < x.at + x.bytes) return true;
+        return false;
+    };
+    auto span = [&](uint32_t id) { const DevBuf& d = t.bufs[id]; return Span{(const char*)d.ptr, d.bytes}; };
+    auto flush = [&]() -> int {
+        if (!pending.held) return ANL_OK;
+        Pending p = std::move(pending);
+        pending = Pending();
+        if (int rc = launch_held(dev, *p.held, nullptr, stream)) { dev->err = "kernel " + std::to_string(p.item) + ": " + dev->err; return rc; }
+        return p.after();
+    };
+    // Is item n a contraction that one writing `writes` may wait for?  What n itself writes is known once it is prepared (its
+    // own output often shares a slot with what the first one reads, and is not stored when a consumer is fused).
+    auto may_wait = [&](size_t n, const std::vector<Span>& writes) {
+        if (!pairs_on || n >= items.size() || absorbed.count(n) || n == tail_split || !items[n].source.empty()) return false;
+        std::shared_ptr<Plan> p;
+        if (get_plan(dev, items[n], opts, p) != ANL_OK || !gemm_holdable(*p)) return false;
+        std::vector<Span> r;
+        for (size_t b = 1; b < items[n].bufs.size(); b++) r.push_back(span(items[n].bufs[b].id));
+        return !meet(writes, r);
+    };
+    // launches `mine`, together with the one that waits if the two go together, or lets it wait for item `next`
+    auto launch_or_hold = [&](size_t i, HeldGemm* mine, std::vector<Span> reads, std::vector<Span> writes, size_t next, std::function<int()> after) -> int {
+        std::unique_ptr<HeldGemm, void (*)(HeldGemm*)> own(mine, drop_held);
+        if (pending.held) {
+            if (gemm_pairs(*pending.held, *own) && !meet(pending.writes, reads) && !meet(pending.writes, writes) && !meet(pending.reads, writes)) {
+                Pending p = std::move(pending);
+                pending = Pending();
+                if (int rc = launch_held(dev, *p.held, own.get(), stream)) { dev->err = "kernel " + std::to_string(i) + ": " + dev->err; return rc; }
+                if (int rc = p.after()) return rc;
+                return after();
+            }
+            if (int rc = flush()) return rc;
+        }
+        pending.held = std::move(own);
+        pending.reads = std::move(reads); pending.writes = std::move(writes); pending.after = std::move(after); pending.item = i;
+        return may_wait(next, pending.writes) ? ANL_OK : flush();
+    };
     for (size_t i = 0; i < items.size(); i++) {
         const Item& it = items[i];
-        if (chains_on && !absorbed.count(i)) {
+        if (absorbed.count(i)) if (int rc = flush()) return rc;
+        if (chains_on && !absorbed.count(i) && !pending.held) {
             size_t used = 0;
             int rc = try_row_chain(dev, items, i, t, stream, &used);
             if (rc != ANL_OK) return rc;
@@ -955,19 +1001,35 @@ int run_items(anl_device* dev, const std::vector<Item>& items, const Bindings& b
                 }
                 cudaEvent_t e0 = nullptr, e1 = nullptr;
                 if (dev->profiling) { cudaEventCreate(&e0); cudaEventCreate(&e1); cudaEventRecord(e0, stream); }
-                int rc = launch_gemm(dev, *plan, ptrs.data(), item_sym(it, binds), stream, 0, -1, &fz, keep_scratch ? &t.owned : nullptr, settled(*plan, ptrs));
+                const bool hold = pairs_on && gemm_holdable(*plan);
+                HeldGemm* mine = nullptr;
+                if (!hold) if (int rc = flush()) return rc;
+                int rc = launch_gemm(dev, *plan, ptrs.data(), item_sym(it, binds), stream, 0, -1, &fz, keep_scratch ? &t.owned : nullptr, settled(*plan, ptrs), hold ? &mine : nullptr);
                 if (dev->profiling) { cudaEventRecord(e1, stream); dev->prof.push_back({e0, e1, KC_GEMM, gemm_flops(*plan, 0)}); }
                 if (rc) { dev->err = "kernel " + std::to_string(i) + ": " + dev->err; return rc; }
-                if (int rc2 = updates_due(i)) return rc2;
-                if (fe) {
-                    dev->stats.epilogues_fused++;
+                if (fe) dev->stats.epilogues_fused++;
+                const bool with_consumer = (bool)fe;
+                auto after = [&, i, with_consumer]() -> int {
+                    if (int rc2 = updates_due(i)) return rc2;
+                    if (!with_consumer) return ANL_OK;
                     // hooks of the consumer, which this launch has just run
                     auto rb = t.after.find(items[i + 1].bufs[0].id);
                     if (rb != t.after.end() && rb->second.allreduce)
                         if (int rc3 = reduce_part(rb->second, 0, rb->second.resident->elems)) return rc3;
-                    if (int rc3 = updates_due(i + 1)) return rc3;
-                    i += 1;
-                }
+                    return updates_due(i + 1);
+                };
+                if (mine) {
+                    std::vector<Span> reads, writes;
+                    for (size_t b = 1; b < it.bufs.size(); b++) reads.push_back(span(it.bufs[b].id));
+                    if (!fe || fz.store_raw) writes.push_back(span(out_id));
+                    if (fe) {
+                        for (size_t b = 1; b < items[i + 1].bufs.size(); b++) if (items[i + 1].bufs[b].id != out_id) reads.push_back(span(items[i + 1].bufs[b].id));
+                        writes.push_back(span(items[i + 1].bufs[0].id));
+                    }
+                    if (partials) writes.push_back(Span{(const char*)partials, (size_t)parts * (size_t)N * 4});
+                    if (int rc2 = launch_or_hold(i, mine, std::move(reads), std::move(writes), i + 1 + (fe ? 1 : 0), after)) return rc2;
+                } else if (int rc2 = after()) return rc2;
+                if (fe) i += 1;
                 continue;
             }
         }
@@ -991,6 +1053,21 @@ int run_items(anl_device* dev, const std::vector<Item>& items, const Bindings& b
             allow_shard = true;
             continue;
         }
+        if (pairs_on && i != tail_split && gemm_holdable(*plan)) {
+            HeldGemm* mine = nullptr;
+            if (int rc = launch_gemm(dev, *plan, ptrs.data(), item_sym(it, binds), stream, 0, -1, nullptr, keep_scratch ? &t.owned : nullptr, settled(*plan, ptrs), &mine)) { dev->err = "kernel " + std::to_string(i) + ": " + dev->err; return rc; }
+            auto after = [&, i]() -> int {
+                auto hook = t.after.find(items[i].bufs[0].id);
+                if (hook != t.after.end() && hook->second.allreduce)
+                    if (int rc = reduce_part(hook->second, 0, hook->second.resident->elems)) return rc;
+                return updates_due(i);
+            };
+            std::vector<Span> reads, writes{span(it.bufs[0].id)};
+            for (size_t b = 1; b < it.bufs.size(); b++) reads.push_back(span(it.bufs[b].id));
+            if (int rc = launch_or_hold(i, mine, std::move(reads), std::move(writes), i + 1, after)) return rc;
+            continue;
+        }
+        if (int rc = flush()) return rc;
         cudaStream_t on = stream;
         if (!gemm_taken(*plan, item_sym(it, binds)) && side_ok(i, ptrs)) { comm_fork(dev, stream); on = dev->comm_stream; dev->stats.side_launches++; }
         if (int rc = launch_plan(dev, *plan, it, ptrs.data(), item_sym(it, binds), on, keep_scratch ? &t.owned : nullptr, settled(*plan, ptrs))) { dev->err = "kernel " + std::to_string(i) + ": " + dev->err; return rc; }
@@ -1000,6 +1077,7 @@ int run_items(anl_device* dev, const std::vector<Item>& items, const Bindings& b
         // ... [update the parameter] once its last reader has been queued as well
         if (int rc = updates_due(i)) return rc;
     }
+    if (int rc = flush()) return rc;
     return comm_join(dev, stream);
 }
 

@@ -210,8 +210,16 @@ int download_f32(anl_device* dev, float* host, const void* src, int dtype, int64
 // hand-written contraction kernels (gemm.cu); returns ANL_OK and fills plan.gemm if the item is a
 // dense SUM-of-products over buffers that they cover, ANL_ERR_UNSUPPORTED otherwise
 int plan_gemm(const Item& item, const GemmTuning& tune, Plan& plan);
+struct HeldGemm;
 int launch_gemm(anl_device* dev, const Plan& plan, void* const* bufs, int64_t sym_value, cudaStream_t stream,
-                int64_t m_begin = 0, int64_t m_end = -1, const GemmFusion* fusion = nullptr, std::vector<void*>* keep_scratch = nullptr, bool b_settled = false);
+                int64_t m_begin = 0, int64_t m_end = -1, const GemmFusion* fusion = nullptr, std::vector<void*>* keep_scratch = nullptr, bool b_settled = false,
+                HeldGemm** hold = nullptr);
+// With `hold`, a plan that is holdable (f16, one-CTA kernel, no operand to copy) is prepared instead of launched; launch_held
+// then launches one, or two whose shapes go together (gemm_pairs) as one kernel.
+bool gemm_holdable(const Plan& plan);
+bool gemm_pairs(const HeldGemm& a, const HeldGemm& b);
+int launch_held(anl_device* dev, HeldGemm& a, HeldGemm* b, cudaStream_t stream);
+void drop_held(HeldGemm* h);
 // parameter number of the operand whose rows are the output's columns (a layer's weights)
 int gemm_b_param(const Plan& plan);
 void launch_hold_stream(cudaStream_t stream, unsigned long long ns);
