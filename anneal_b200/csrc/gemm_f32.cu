@@ -381,36 +381,64 @@ gemm_f32_few_rows_axpy(const float* __restrict__ a, const float* __restrict__ b,
     cluster.sync();               // the other CTAs' shared memory stays until the first has read it
 }
 
-// D[m, n] = sum_k A[k, m] * B[k, n] with few terms (a weight gradient at a small batch): every thread
-// four consecutive columns of one row, the terms added in ascending k like the reference's loop.
-// U terms' loads are in flight: one by one, 64 terms and 128 x 784 outputs took 16.3 us of a step that went from 37.6 to
-// 32.8 with this and the generated reductions' loops unrolled; with fewer than eight terms the plain loop is the
-// shorter one (one term, 1024 x 4096 outputs twice a step: 41.6 us a step against 45.6).
-template <int U>
-__global__ void __launch_bounds__(256) gemm_f32_few_terms(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ d,
-                                                           int M, int N, int K, long long a_sk, long long b_sk, int ldd, int vec) {
+// D[m, n] = sum_k A[k, m] * B[k, n] with few terms (a weight gradient at a small batch), the terms added in ascending k like the
+// reference's loop.  A thread has R rows of four consecutive columns, a block R * 4 rows of 128, and the loads of U terms are in
+// flight together, the last few as well.
+//   many outputs   R = 4, U = 4: with one row a thread every four products took a load of each operand, and the loads were the
+//                  bound, as were 64-bit divisions for the thread's place (alone, 6 us of events included: 1024 x 4096 x 32 30.8 -> 18.4 us,
+//                  4096 x 1024 x 64 54.1 -> 28.8, five terms 13.3 -> 10.2; a symbolic step with one row, two of these, 33.0 -> 30.9)
+//   few outputs    R = 1, U = 16: the bound is the chain of latencies, one for every U terms (128 x 784 x 64 12.3 -> 10.3)
+constexpr int FT_COLS = 128, FT_ROWS = 4, FT_THREADS = 128;
+template <int R, int U>
+__global__ void __launch_bounds__(FT_THREADS) gemm_f32_few_terms(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ d,
+                                                                  int M, int N, int K, long long a_sk, long long b_sk, int ldd, int col_blocks, int vec_a, int vec_b) {
     enter_kernel();
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int n4 = (N + 3) / 4;
-    const long long m = t / n4;
-    const int n = (int)(t % n4) * 4;
-    if (m >= M) return;
-    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll U
-    for (int k = 0; k < K; k++) {
-        const float av = a[(long long)k * a_sk + m];
-        const float* brow = b + (long long)k * b_sk + n;
-        if (vec) {
-            const float4 bv = *reinterpret_cast<const float4*>(brow);
-            acc[0] = fmaf(av, bv.x, acc[0]); acc[1] = fmaf(av, bv.y, acc[1]); acc[2] = fmaf(av, bv.z, acc[2]); acc[3] = fmaf(av, bv.w, acc[3]);
-        } else {
+    const int by = (int)(blockIdx.x / (unsigned)col_blocks), bx = (int)blockIdx.x - by * col_blocks;
+    const int n = bx * FT_COLS + (threadIdx.x & 31) * 4, m = (by * FT_ROWS + (threadIdx.x >> 5)) * R;
+    if (n >= N || m >= M) return;
+    float acc[R][4];
 #pragma unroll
-            for (int j = 0; j < 4; j++) if (n + j < N) acc[j] = fmaf(av, brow[j], acc[j]);
+    for (int r = 0; r < R; r++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[r][j] = 0.0f;
+    for (int k0 = 0; k0 < K; k0 += U) {
+        float av[U][R], bv[U][4];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const bool on = k0 + u < K;
+            const float* const ap = a + (long long)(k0 + u) * a_sk + m;
+            const float* const bp = b + (long long)(k0 + u) * b_sk + n;
+            if (R == 4 && vec_a) {
+                const float4 v = on ? *reinterpret_cast<const float4*>(ap) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                av[u][0] = v.x; av[u][1 % R] = v.y; av[u][2 % R] = v.z; av[u][3 % R] = v.w;
+            } else {
+#pragma unroll
+                for (int r = 0; r < R; r++) av[u][r] = on && m + r < M ? ap[r] : 0.0f;
+            }
+            if (vec_b) {
+                const float4 v = on ? *reinterpret_cast<const float4*>(bp) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                bv[u][0] = v.x; bv[u][1] = v.y; bv[u][2] = v.z; bv[u][3] = v.w;
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; j++) bv[u][j] = on && n + j < N ? bp[j] : 0.0f;
+            }
         }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (k0 + u < K) {
+#pragma unroll
+                for (int r = 0; r < R; r++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) acc[r][j] = fmaf(av[u][r], bv[u][j], acc[r][j]);
+            }
     }
-    float* out = d + m * ldd + n;
-    if (vec) *reinterpret_cast<float4*>(out) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-    else for (int j = 0; j < 4; j++) if (n + j < N) out[j] = acc[j];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        if (m + r >= M) break;
+        float* const out = d + (long long)(m + r) * ldd + n;
+        if (vec_b) *reinterpret_cast<float4*>(out) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+        else for (int j = 0; j < 4; j++) if (n + j < N) out[j] = acc[r][j];
+    }
 }
 
 // Which hand-written kernel, if any, finishes a contraction of these extents and strides sooner than
@@ -471,10 +499,17 @@ int launch_gemm_f32(anl_device* dev, const float* a, const float* b, float* d, i
 #undef ANL_AXPY
         }
         else {
-            const int vec4 = (N % 4 == 0) && (b_sk % 4 == 0) && (((uintptr_t)b & 15) == 0) && (((uintptr_t)d & 15) == 0);
-            const long long threads = M * ((N + 3) / 4);
-            const unsigned blocks = (unsigned)((threads + 255) / 256);
-            le = launch_static(dev, K >= 8 ? gemm_f32_few_terms<8> : gemm_f32_few_terms<1>, dim3(blocks), dim3(256), stream, 1, a, b, d, (int)M, (int)N, (int)K, a_sk, b_sk, (int)N, vec4);
+            const int vec_b = N % 4 == 0 && b_sk % 4 == 0 && al16(b) && al16(d), vec_a = M % 4 == 0 && a_sk % 4 == 0 && al16(a);
+            const int64_t col_blocks = (N + FT_COLS - 1) / FT_COLS;
+            // four rows a thread from two blocks an SM on
+            const bool many = col_blocks * ((M + 4 * FT_ROWS - 1) / (4 * FT_ROWS)) >= 2 * dev->prop.multiProcessorCount;
+            const int64_t blocks = col_blocks * ((M + FT_ROWS * (many ? 4 : 1) - 1) / (FT_ROWS * (many ? 4 : 1)));
+            if (blocks > 0x7fffffffLL) return dev->fail(ANL_ERR_LIMIT, "gemm f32: grid too large");
+#define ANL_FT(R, U) le = launch_static(dev, gemm_f32_few_terms<R, U>, dim3((unsigned)blocks), dim3(FT_THREADS), stream, 1, a, b, d, (int)M, (int)N, (int)K, a_sk, b_sk, (int)N, (int)col_blocks, vec_a, vec_b)
+            if (many) { if (K == 1) ANL_FT(4, 1); else ANL_FT(4, 4); }
+            else if (K > 8) ANL_FT(1, 16);
+            else ANL_FT(1, 8);
+#undef ANL_FT
         }
         if (le != cudaSuccess) return dev->fail(ANL_ERR_CUDA, std::string("gemm f32: launch: ") + cudaGetErrorString(le));
         dev->stats.kernels_launched++;
