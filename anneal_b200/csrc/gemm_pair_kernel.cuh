@@ -504,11 +504,7 @@ gemm_f16_tcgen05_pair(const __grid_constant__ TensorMap map_a, const __grid_cons
             tile_of(tt, tiles_m, g.tiles_n, g.full_tiles, tm, n0, width);
             const int m0 = tm * (2 * BM) + (int)rank * BM;
             const int row = m0 + quad * 32 + lane;
-            #if CFG_TF32
-            const size_t row_off = (size_t)row * g.ldd + (size_t)sp * (size_t)g.split_stride;
-#else
-            const size_t row_off = (size_t)row * g.ldd;
-#endif
+            const size_t row_off = (size_t)row * g.ldd; (void)row_off;
             const bool row_ok = row < g.M;
             const bool vec_ok = (g.ldd % 8 == 0); (void)vec_ok;
             const int c_begin = col_half * (width / 64), c_end = c_begin + width / 64;      // this warp's 32-column chunks
@@ -523,6 +519,71 @@ gemm_f16_tcgen05_pair(const __grid_constant__ TensorMap map_a, const __grid_cons
             for (int q = 0; q < 4; q++)
                 if (urow0 + q < g.M && n0 + c_begin * 32 + ucol < g.N) epi8_load_(urow0 + q, n0 + c_begin * 32 + ucol, g.ep, raw_next[q]);
 #endif
+#if CFG_TF32
+            // f32 result of each chunk of k: stored, or added to the sum of the chunks before it.  Groups of four lanes exchange
+            // 16-byte pieces as the f16 form does, so that an instruction touches 8 rows x 64 contiguous bytes; as rows of their own
+            // 32 lanes touched half a sector each (4096 x 1024 x 2048 alone, with the operand splits, 107.5 -> 101.4 us; 1024 x 4096 x 256
+            // 29.7 -> 26.6; 4096-cubed 578 -> 566).
+            float* const d = reinterpret_cast<float*>(g.d_raw) + (size_t)sp * (size_t)g.split_stride;
+            const int pcol0 = n0 + 4 * (lane & 3);
+            for (int ch = 0; ch < chunks; ch++) {
+                if (!mbar_wait(smem_u32(&acc_full[acc]), acc_phase, &failed)) { ok = false; if (lane == 0) { *(volatile int*)g.status = 14; failed = 1; } break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+                for (int c = c_begin; c < c_end; c++) {
+                    unsigned v[32];
+                    tmem_ld32(tmem_base + ((unsigned)(quad * 32) << 16) + acc * BNT + c * 32, v);
+                    float4 o[2][4];
+                    const bool vec = (g.ldd & 3) == 0;
+                    if (ch > 0 && vec) {
+#pragma unroll
+                        for (int h = 0; h < 2; h++)
+#pragma unroll
+                            for (int q = 0; q < 4; q++)
+                                if (urow0 + q < g.M && pcol0 + c * 32 + 16 * h < g.N) o[h][q] = *reinterpret_cast<const float4*>(d + (size_t)(urow0 + q) * g.ldd + pcol0 + c * 32 + 16 * h);
+                    }
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (n0 + c * 32 >= g.N) continue;          // warp-uniform
+                    if (vec) {
+                        const bool b0 = (lane & 1) != 0, b1 = (lane & 2) != 0;
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            uint4 Q[4], A[2][2], T[4];
+#pragma unroll
+                            for (int k = 0; k < 4; k++) Q[k] = make_uint4(v[16 * h + 4 * k], v[16 * h + 4 * k + 1], v[16 * h + 4 * k + 2], v[16 * h + 4 * k + 3]);
+#pragma unroll
+                            for (int k = 0; k < 2; k++) {
+                                const uint4 got = shfl_xor_u4(sel_u4(b0, Q[2 * k], Q[2 * k + 1]), 1), keep = sel_u4(b0, Q[2 * k + 1], Q[2 * k]);
+                                A[k][0] = sel_u4(b0, got, keep);
+                                A[k][1] = sel_u4(b0, keep, got);
+                            }
+#pragma unroll
+                            for (int j = 0; j < 2; j++) {
+                                const uint4 got = shfl_xor_u4(sel_u4(b1, A[0][j], A[1][j]), 2), keep = sel_u4(b1, A[1][j], A[0][j]);
+                                T[j] = sel_u4(b1, got, keep);
+                                T[2 + j] = sel_u4(b1, keep, got);
+                            }
+#pragma unroll
+                            for (int q = 0; q < 4; q++) {
+                                if (urow0 + q >= g.M || pcol0 + c * 32 + 16 * h >= g.N) continue;
+                                float4 r = make_float4(__uint_as_float(T[q].x), __uint_as_float(T[q].y), __uint_as_float(T[q].z), __uint_as_float(T[q].w));
+                                if (ch > 0) { r.x = o[h][q].x + r.x; r.y = o[h][q].y + r.y; r.z = o[h][q].z + r.z; r.w = o[h][q].w + r.w; }
+                                *reinterpret_cast<float4*>(d + (size_t)(urow0 + q) * g.ldd + pcol0 + c * 32 + 16 * h) = r;
+                            }
+                        }
+                    } else if (row_ok) {
+                        float* const out = d + (size_t)row * g.ldd + n0 + c * 32;
+#pragma unroll
+                        for (int j = 0; j < 32; j++)
+                            if (n0 + c * 32 + j < g.N) out[j] = (ch > 0) ? out[j] + __uint_as_float(v[j]) : __uint_as_float(v[j]);
+                    }
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[acc]), 0));   // the leader waits for both CTAs' epilogues
+                if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+            }
+#else
             for (int ch = 0; ch < chunks; ch++) {
             if (!mbar_wait(smem_u32(&acc_full[acc]), acc_phase, &failed)) { ok = false; if (lane == 0) { *(volatile int*)g.status = 14; failed = 1; } break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -547,24 +608,6 @@ gemm_f16_tcgen05_pair(const __grid_constant__ TensorMap map_a, const __grid_cons
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 const int col = n0 + c * 32;
                 if (col >= g.N) continue;                  // warp-uniform
-#if CFG_TF32
-                // f32 result of this chunk of k: stored, or added to the sum of the chunks before it
-                if (row_ok) {
-                    float* out = reinterpret_cast<float*>(g.d_raw) + row_off + col;
-                    if ((g.ldd & 3) == 0 && col + 32 <= g.N) {
-#pragma unroll
-                        for (int q = 0; q < 8; q++) {
-                            float4 r = make_float4(__uint_as_float(v[4 * q]), __uint_as_float(v[4 * q + 1]), __uint_as_float(v[4 * q + 2]), __uint_as_float(v[4 * q + 3]));
-                            if ((ch > 0)) { const float4 o = *reinterpret_cast<const float4*>(out + 4 * q); r.x = o.x + r.x; r.y = o.y + r.y; r.z = o.z + r.z; r.w = o.w + r.w; }
-                            *reinterpret_cast<float4*>(out + 4 * q) = r;
-                        }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 32; j++)
-                            if (col + j < g.N) out[j] = (ch > 0) ? out[j] + __uint_as_float(v[j]) : __uint_as_float(v[j]);
-                    }
-                }
-#else
                 // the single narrowing of the f32 accumulator
                 __half2 h[16];
 #pragma unroll
@@ -629,13 +672,13 @@ gemm_f16_tcgen05_pair(const __grid_constant__ TensorMap map_a, const __grid_cons
                         if (col + 2 * j + 1 < g.N) d_raw[row_off + col + 2 * j + 1] = __high2half(h[j]);
                     }
                 }
-#endif
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[acc]), 0));   // the leader waits for both CTAs' epilogues
             if (++acc == 2) { acc = 0; acc_phase ^= 1; }
             }
+#endif
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
