@@ -426,6 +426,7 @@ int launch_sgd(anl_device* dev, anl_buffer* master, anl_buffer* param, anl_buffe
 // one copy: each copy from or to pageable memory is a call of its own that stages, waits and returns.  The f32 MLP step at
 // batch 64 (eight leaves and five outputs, 1 MB in all) went from 370 to 208 us, with the parsed schedule kept as well.  Above it the staging copy costs more than the calls.
 constexpr size_t kHostStageMax = (size_t)8 << 20;
+constexpr size_t kHostStagePiece = (size_t)128 << 10;      // staged leaves are sent on in pieces of at least this
 
 // Makes the pinned block hold `bytes`, before a call queues anything of its own: every call that fills the block waits for
 // the stream before it returns, so it is free then, and what earlier calls left queued (replays, with their
@@ -588,8 +589,17 @@ int build_table(anl_device* dev, const std::vector<Item>& items, const Bindings&
         char* const stage = (char*)dev->host_stage;
         if (int rc = dev->alloc(leaf_bytes, (void**)&leaf_block)) return rc;
         t.owned.push_back(leaf_block);
-        for (const Leaf& l : leaves) { std::memcpy(stage + l.at, l.data, l.bytes); dev->stats.h2d_bytes += l.bytes; }
-        CK(dev, cudaMemcpyAsync(leaf_block, stage, leaf_bytes, cudaMemcpyHostToDevice, dev->stream));
+        // what has been staged travels while the next leaves are staged
+        size_t sent = 0;
+        for (size_t k = 0; k < leaves.size(); k++) {
+            const Leaf& l = leaves[k];
+            std::memcpy(stage + l.at, l.data, l.bytes);
+            dev->stats.h2d_bytes += l.bytes;
+            const size_t upto = k + 1 < leaves.size() ? leaves[k + 1].at : leaf_bytes;
+            if (upto - sent < kHostStagePiece && k + 1 < leaves.size()) continue;
+            CK(dev, cudaMemcpyAsync(leaf_block + sent, stage + sent, upto - sent, cudaMemcpyHostToDevice, dev->stream));
+            sent = upto;
+        }
     }
     for (auto& it : items) {
         int64_t sym = item_sym(it, binds);
