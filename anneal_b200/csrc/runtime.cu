@@ -853,22 +853,27 @@ int run_items(anl_device* dev, const std::vector<Item>& items, const Bindings& b
         }
         return true;
     };
-    // Inside a captured graph: memory that no kernel of the schedule writes (a layer's weights; their updates come after
-    // their last reader) holds its values from the start of the replay on.
-    std::set<const void*> written;
-    if (keep_scratch) for (auto& it : items) written.insert(t.bufs[it.bufs[0].id].ptr);
-    auto settled = [&](const Plan& p, const std::vector<void*>& ptrs) { return keep_scratch && gemm_fusable(p) && !written.count(ptrs[gemm_b_param(p)]); };
-    // Two contractions in a row that do not depend on each other (a layer's weight gradient, then the gradient of its input)
-    // are one launch where both are small (gemm_small_kernel.cuh): the first waits here, prepared, until the second is.
-    // Only when the very next item is such a contraction, so that nothing is launched between them.
     struct Span { const char* at; size_t bytes; };
-    struct Pending { std::unique_ptr<HeldGemm, void (*)(HeldGemm*)> held{nullptr, drop_held}; std::vector<Span> reads, writes; std::function<int()> after; size_t item = 0; } pending;
-    const bool pairs_on = dev->nranks <= 1 && !dev->profiling && !(dev->flags & ANL_OPEN_BEAM);
     auto meet = [](const std::vector<Span>& a, const std::vector<Span>& b) {
         for (const Span& x : a) for (const Span& y : b) if (x.at < y.at + y.bytes && y.at < x.at + x.bytes) return true;
         return false;
     };
     auto span = [&](uint32_t id) { const DevBuf& d = t.bufs[id]; return Span{(const char*)d.ptr, d.bytes}; };
+    // Inside a captured graph: an operand that no kernel of the schedule writes (a layer's weights; their updates come after
+    // their last reader) holds its values from the start of the replay on.  Asked by buffer, as an output may move to other
+    // memory below, and by the memory that the outputs have here, as a caller may place an output over an input.
+    std::vector<Span> written;
+    if (keep_scratch) for (auto& it : items) written.push_back(span(it.bufs[0].id));
+    auto settled = [&](const Plan& p, const Item& it) {
+        if (!keep_scratch || !gemm_fusable(p)) return false;
+        const uint32_t b = it.bufs[gemm_b_param(p)].id;
+        return !t.written.count(b) && !meet(written, {span(b)});
+    };
+    // Two contractions in a row that do not depend on each other (a layer's weight gradient, then the gradient of its input)
+    // are one launch where both are small (gemm_small_kernel.cuh): the first waits here, prepared, until the second is.
+    // Only when the very next item is such a contraction, so that nothing is launched between them.
+    struct Pending { std::unique_ptr<HeldGemm, void (*)(HeldGemm*)> held{nullptr, drop_held}; std::vector<Span> reads, writes; std::function<int()> after; size_t item = 0; } pending;
+    const bool pairs_on = dev->nranks <= 1 && !dev->profiling && !(dev->flags & ANL_OPEN_BEAM);
     auto flush = [&]() -> int {
         if (!pending.held) return ANL_OK;
         Pending p = std::move(pending);
@@ -1014,7 +1019,7 @@ int run_items(anl_device* dev, const std::vector<Item>& items, const Bindings& b
                 const bool hold = pairs_on && gemm_holdable(*plan);
                 HeldGemm* mine = nullptr;
                 if (!hold) if (int rc = flush()) return rc;
-                int rc = launch_gemm(dev, *plan, ptrs.data(), item_sym(it, binds), stream, 0, -1, &fz, keep_scratch ? &t.owned : nullptr, settled(*plan, ptrs), hold ? &mine : nullptr);
+                int rc = launch_gemm(dev, *plan, ptrs.data(), item_sym(it, binds), stream, 0, -1, &fz, keep_scratch ? &t.owned : nullptr, settled(*plan, it), hold ? &mine : nullptr);
                 if (dev->profiling) { cudaEventRecord(e1, stream); dev->prof.push_back({e0, e1, KC_GEMM, gemm_flops(*plan, 0)}); }
                 if (rc) { dev->err = "kernel " + std::to_string(i) + ": " + dev->err; return rc; }
                 if (fe) dev->stats.epilogues_fused++;
@@ -1065,7 +1070,7 @@ int run_items(anl_device* dev, const std::vector<Item>& items, const Bindings& b
         }
         if (pairs_on && i != tail_split && gemm_holdable(*plan)) {
             HeldGemm* mine = nullptr;
-            if (int rc = launch_gemm(dev, *plan, ptrs.data(), item_sym(it, binds), stream, 0, -1, nullptr, keep_scratch ? &t.owned : nullptr, settled(*plan, ptrs), &mine)) { dev->err = "kernel " + std::to_string(i) + ": " + dev->err; return rc; }
+            if (int rc = launch_gemm(dev, *plan, ptrs.data(), item_sym(it, binds), stream, 0, -1, nullptr, keep_scratch ? &t.owned : nullptr, settled(*plan, it), &mine)) { dev->err = "kernel " + std::to_string(i) + ": " + dev->err; return rc; }
             auto after = [&, i]() -> int {
                 auto hook = t.after.find(items[i].bufs[0].id);
                 if (hook != t.after.end() && hook->second.allreduce)
@@ -1080,7 +1085,7 @@ int run_items(anl_device* dev, const std::vector<Item>& items, const Bindings& b
         if (int rc = flush()) return rc;
         cudaStream_t on = stream;
         if (!gemm_taken(*plan, item_sym(it, binds)) && side_ok(i, ptrs)) { comm_fork(dev, stream); on = dev->comm_stream; dev->stats.side_launches++; }
-        if (int rc = launch_plan(dev, *plan, it, ptrs.data(), item_sym(it, binds), on, keep_scratch ? &t.owned : nullptr, settled(*plan, ptrs))) { dev->err = "kernel " + std::to_string(i) + ": " + dev->err; return rc; }
+        if (int rc = launch_plan(dev, *plan, it, ptrs.data(), item_sym(it, binds), on, keep_scratch ? &t.owned : nullptr, settled(*plan, it))) { dev->err = "kernel " + std::to_string(i) + ": " + dev->err; return rc; }
         // side stream: [all-reduce this gradient] behind the producing kernel ...
         if (ra != t.after.end() && ra->second.allreduce)
             if (int rc = reduce_part(ra->second, 0, ra->second.resident->elems)) return rc;
