@@ -332,10 +332,9 @@ SmallVariant choose_small(int64_t M, int64_t N, int64_t K, bool a_mn, bool b_mn,
             // land two CTAs to an SM even where there are SMs to spare, and clusters that do not all fit
             // at once start late (512 x 4096 x 4096 split four ways: 39 us against 22.6 split two ways).
             const bool alone = tf32 && nt == 128 && v.prows == 128;         // 64 KB a stage: one CTA an SM
-            const bool eight_alone = tf32 && splits == 8 && ctas <= 64;      // f32 CTAs of 200 KB: half of the SMs take one each
-            const double n = std::max(std::ceil(ctas / 148.0), splits == 8 && !eight_alone ? 2.0 : 1.0);
-            const double load = std::max(n * per * (double)(parts * (v.prows + nt) * 128) / (n > 1 && !alone ? 135e3 : 100e3), std::ceil(alone ? n : n / 2) * per * (tf32 ? 0.5 : 0.25));
-            double t = 3.0 + load + (splits == 1 ? 0.0 : splits == 2 ? 2.0 : splits == 4 ? 2.5 : eight_alone ? 4.0 : 7.0);
+            const double n = std::max(std::ceil(ctas / 148.0), splits == 8 ? 2.0 : 1.0);
+            const double load = std::max(n * per * (double)(parts * (v.prows + nt) * 128) / (n > 1 && !alone ? 135e3 : 100e3), std::ceil(alone ? n : n / 2) * per * 0.25);
+            double t = 3.0 + load + (splits == 1 ? 0.0 : splits == 2 ? 2.0 : splits == 4 ? 2.5 : 7.0);
             if (splits > 1 && ctas > 2 * 148) t *= 2;
             if (t < best) { best = t; best_ctas = ctas; v.nt = nt; v.splits = splits; v.chunk = per > most ? most : 0; }
         }
