@@ -2094,7 +2094,7 @@ struct Gen {
         } else k << "  long long g = (long long)blockIdx.x * TOUTS + grp;\n";
         k << "  const bool valid = g < " << total_expr() << ";\n";
         k << "  if (!valid) g = " << total_expr() << " - 1;\n";
-        std::string at = "g";
+        std::string at = "g";                   // place of this thread's output
         if (!enum_reduce.empty() && lanes == 1 && !split_mode && !has_sym) {
             const std::vector<int> order = thread_order(), natural = loop_ranges;
             if (order != natural) {
@@ -2113,7 +2113,7 @@ struct Gen {
             k << top.code;
             k << "  if (valid && lane == 0) data0[" << at << "] = " << store_value(v, body) << ";\n";
         } else {
-            if (!emit_cases(k, "  if (valid && lane == 0) data0[g] = ")) return false;
+            if (!emit_cases(k, "  if (valid && lane == 0) data0[" + at + "] = ")) return false;
         }
         k << "}\n";
         out.klass = split_mode ? KC_REDUCE_SPLIT : KC_REDUCE;
