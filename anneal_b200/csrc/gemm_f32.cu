@@ -382,20 +382,23 @@ gemm_f32_few_rows_axpy(const float* __restrict__ a, const float* __restrict__ b,
 }
 
 // D[m, n] = sum_k A[k, m] * B[k, n] with few terms (a weight gradient at a small batch), the terms added in ascending k like the
-// reference's loop.  A thread has R rows of four consecutive columns, a block R * 4 rows of 128, and the loads of U terms are in
-// flight together, the last few as well.
+// reference's loop.  A thread has R rows of four consecutive columns, and the loads of U terms are in flight together, the last
+// few as well; threads run through the rows, so that no lane is idle where 128 does not divide the columns.
 //   many outputs   R = 4, U = 4: with one row a thread every four products took a load of each operand, and the loads were the
-//                  bound, as were 64-bit divisions for the thread's place (alone, 6 us of events included: 1024 x 4096 x 32 30.8 -> 18.4 us,
-//                  4096 x 1024 x 64 54.1 -> 28.8, five terms 13.3 -> 10.2; a symbolic step with one row, two of these, 33.0 -> 30.9)
-//   few outputs    R = 1, U = 16: the bound is the chain of latencies, one for every U terms (128 x 784 x 64 12.3 -> 10.3)
-constexpr int FT_COLS = 128, FT_ROWS = 4, FT_THREADS = 128;
+//                  bound, as were 64-bit divisions for the thread's place.  us a launch, 16 of them in a row, one row a thread
+//                  against four: 1024 x 2048 outputs of 64 terms 25.4 -> 14.9, 400 x 700 9.6 -> 6.9, 3000 x 70 14.3 -> 8.0
+//   few outputs    R = 2, U = 8: the bound is the chain of latencies, one for every U terms, and more loads a thread leave room
+//                  for fewer threads (sixteen terms of one row: from four blocks an SM on a second wave, 700 x 131 x 64 11.0).
+//                  128 x 1000 x 64 7.4 -> 6.0, 700 x 131 x 64 11.6 -> 7.1, 520 x 132 x 24 3.4 -> 2.9
+constexpr int FT_THREADS = 128;
 template <int R, int U>
 __global__ void __launch_bounds__(FT_THREADS) gemm_f32_few_terms(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ d,
-                                                                  int M, int N, int K, long long a_sk, long long b_sk, int ldd, int col_blocks, int vec_a, int vec_b) {
+                                                                  int M, int N, int K, long long a_sk, long long b_sk, int ldd, unsigned groups, int vec_a, int vec_b) {
     enter_kernel();
-    const int by = (int)(blockIdx.x / (unsigned)col_blocks), bx = (int)blockIdx.x - by * col_blocks;
-    const int n = bx * FT_COLS + (threadIdx.x & 31) * 4, m = (by * FT_ROWS + (threadIdx.x >> 5)) * R;
-    if (n >= N || m >= M) return;
+    // fours of columns, then groups of R rows: fewer than 2^32 in all
+    const unsigned t = blockIdx.x * FT_THREADS + threadIdx.x, n4 = ((unsigned)N + 3) / 4, group = t / n4;
+    if (group >= groups) return;
+    const int n = (int)(t - group * n4) * 4, m = (int)(group * R);
     float acc[R][4];
 #pragma unroll
     for (int r = 0; r < R; r++)
@@ -500,15 +503,17 @@ int launch_gemm_f32(anl_device* dev, const float* a, const float* b, float* d, i
         }
         else {
             const int vec_b = N % 4 == 0 && b_sk % 4 == 0 && al16(b) && al16(d), vec_a = M % 4 == 0 && a_sk % 4 == 0 && al16(a);
-            const int64_t col_blocks = (N + FT_COLS - 1) / FT_COLS;
-            // four rows a thread from two blocks an SM on
-            const bool many = col_blocks * ((M + 4 * FT_ROWS - 1) / (4 * FT_ROWS)) >= 2 * dev->prop.multiProcessorCount;
-            const int64_t blocks = col_blocks * ((M + FT_ROWS * (many ? 4 : 1) - 1) / (FT_ROWS * (many ? 4 : 1)));
-            if (blocks > 0x7fffffffLL) return dev->fail(ANL_ERR_LIMIT, "gemm f32: grid too large");
-#define ANL_FT(R, U) le = launch_static(dev, gemm_f32_few_terms<R, U>, dim3((unsigned)blocks), dim3(FT_THREADS), stream, 1, a, b, d, (int)M, (int)N, (int)K, a_sk, b_sk, (int)N, (int)col_blocks, vec_a, vec_b)
-            if (many) { if (K == 1) ANL_FT(4, 1); else ANL_FT(4, 4); }
-            else if (K > 8) ANL_FT(1, 16);
-            else ANL_FT(1, 8);
+            // Four rows a thread where that leaves two blocks for every three SMs: 3000 x 70 x 64 (106 blocks) 8.0 us against 9.8
+            // with two rows, 400 x 700 x 64 (137) 6.9 against 8.8; 128 x 1000 x 64 (63) 6.5 against 6.0, 700 x 131 x 64 (46) 8.0
+            // against 7.1.  One and two terms of many outputs, bound by writing them, one at a time: 1024 x 999 x 2 3.5 against 3.8.
+            const int64_t n4 = (N + 3) / 4;
+            const int rows = 3 * ((M + 3) / 4 * n4) >= 2 * (int64_t)FT_THREADS * dev->prop.multiProcessorCount ? 4 : 2;
+            const int64_t groups = (M + rows - 1) / rows, blocks = (groups * n4 + FT_THREADS - 1) / FT_THREADS;
+            if (blocks * FT_THREADS >= (1ll << 32)) return dev->fail(ANL_ERR_LIMIT, "gemm f32: grid too large");
+#define ANL_FT(R, U) le = launch_static(dev, gemm_f32_few_terms<R, U>, dim3((unsigned)blocks), dim3(FT_THREADS), stream, 1, a, b, d, (int)M, (int)N, (int)K, a_sk, b_sk, (int)N, (unsigned)groups, vec_a, vec_b)
+            if (rows == 2) ANL_FT(2, 8);
+            else if (K <= 2) ANL_FT(4, 1);
+            else ANL_FT(4, 4);
 #undef ANL_FT
         }
         if (le != cudaSuccess) return dev->fail(ANL_ERR_CUDA, std::string("gemm f32: launch: ") + cudaGetErrorString(le));

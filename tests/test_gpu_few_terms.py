@@ -27,3 +27,10 @@ def test_few_terms(cuda, M, N, K):
     # K products added one after the other in f32: K roundings of at most half a unit of the partial sums
     bound = (K + 1) * 2.0 ** -24 * (np.abs(am[:, rows]).T @ np.abs(bm))
     assert (np.abs(y[rows] - ref) <= bound + 1e-30).all()
+
+
+# two and four rows a thread on either side of the line (66 and 99 to 101 blocks of four rows); warps that hold the end of one
+# row and the start of the next; one column group a row; a last group of one, two and three rows
+@pytest.mark.parametrize("M,N,K", [(128, 1056, 8), (132, 1056, 9), (401, 505, 24), (402, 511, 3), (3000, 70, 9), (1021, 65, 64), (1025, 64, 2), (400, 700, 17), (65537, 64, 4), (66, 65536, 2)])
+def test_threads_run_through_the_rows(cuda, M, N, K):
+    test_few_terms(cuda, M, N, K)
