@@ -1935,11 +1935,20 @@ struct Gen {
         auto fix_all = [&](const std::vector<int>& rs, int64_t v) { for (size_t e = rs.size(); e-- > 0;) { fix_range(rs[e], v % N(rs[e]).arg); v /= N(rs[e]).arg; } };
         int64_t cases = 1;
         for (int r : outer) cases *= N(r).arg;
-        // blocks of up to 1024 lanes an output group; with few groups, parts of four trips a lane or more in several blocks
+        // Many groups: a block of up to 1024 lanes each.  Few: parts of one trip a lane in up to 16 blocks a group, from
+        // three trips on wider blocks and then more of them while the SMs have room, as a block's trips are one chain of
+        // latencies; one block where a lane of it has a trip or two, as the ticket and the second pass cost as much.  us a launch in a row of sixteen, groups x
+        // terms, a block per output (no such form) | parts of four trips a lane | this: 4 x 1200 4.0 | 6.1 | 4.1, 6 x 2000 5.8 | 6.9 | 4.0,
+        // 8 x 2048 5.4 | 5.8 | 3.8, 8 x 6272 13.5 | 6.9 | 4.9, 8 x 25088 20 | 8.6 | 7.5, 4 x 73728 18.5 | 9.8 | 9.8, 64 x 18432 62 | 18 | 14;
+        // in one block 64 x 1152 4.8 | 5.8 | 4.1, 4 x 1024 3.8 | 3.9 | 3.4.
         const int64_t groups = static_total() / ninner;
         int L = 256, parts = 1;
         if (groups >= 74) { while (L < 1024 && groups * L < 148 * 1024 && rmax / (L * 2) >= 4) L *= 2; }
-        else parts = (int)std::max<int64_t>(1, std::min<int64_t>({(rmax + L * 4 - 1) / (L * 4), 148 * 2 / groups, 1024}));
+        else if (rmax <= (groups >= 32 ? 1280 : 1024)) L = 1024;
+        else {
+            parts = (int)std::min<int64_t>({(rmax + L - 1) / L, 512 / groups, 16});
+            while (groups * parts * L * 2 <= 148 * 1024 && rmax > 3ll * L * parts) { if (L < 1024) L *= 2; else parts *= 2; }
+        }
         if (groups > kMaxTickets && parts > 1) parts = 1;
         rc_layout = true; lanes = threads = L; touts = 1;
 
