@@ -453,6 +453,21 @@ int gemm_small_parts(const Plan& plan) {
     return v.splits * (v.chunk ? 2 : 1);
 }
 
+// Is a consumer worth joining where its output has to move for it (run_items)?  Not where one wave of large tiles leaves the whole
+// finish exposed: us a layer with GELU, joined against apart, two-CTA kernel 706 x 3840 (45 tiles for 74 pairs) +1.0, 1024 x 3840
+// (60) +0.6, 1500 x 3840 (90) -2.8; one-CTA kernel, 128 x 128 tiles of whole K on an SM each, 2048 x 1024 +0.3, 1500 x 1024 0.0;
+// narrower ones 1024 x 1024 -0.8, 512 x 512 -0.9, split ones 384 x 1024 -1.9.
+bool gemm_joins_moved(anl_device* dev, const Plan& plan) {
+    const Contraction& c = plan.gemm->c;
+    if (small_takes(*plan.gemm, c.M)) {
+        const SmallVariant v = choose_small(*plan.gemm, c.M);
+        const int64_t tiles = ((c.M + BM - 1) / BM) * ((c.N + v.nt - 1) / v.nt);
+        return v.splits > 1 || v.nt < 128 || v.prows < 128 || tiles > gemm_sm_budget(dev);
+    }
+    const PairVariant v = choose_variant(dev, *plan.gemm, c.M);
+    return ((c.M + 2 * BM - 1) / (2 * BM)) * ((c.N + v.bnt - 1) / v.bnt) > gemm_sm_budget(dev) / 2;
+}
+
 // the source that a launch of this plan will use, and the kernel itself
 int gemm_source(anl_device* dev, const Plan& plan, const std::string& epilogue, std::string& out) {
     if (!gemm_fusable(plan)) return ANL_ERR_UNSUPPORTED;

@@ -971,12 +971,13 @@ int run_items(anl_device* dev, const std::vector<Item>& items, const Bindings& b
                     // The consumer's output must not live in memory this contraction still reads: the planner, for which the
                     // contraction is over when its consumer starts, gives every second layer of a forward pass its input's
                     // slot.  Such an output moves to a block of its own (a launch of 2.7 us and a round trip of the
-                    // activations saved, 32 x 4096 in f16); without one, and where it is not a slot, the two stay apart.
+                    // activations saved, 32 x 4096 in f16); without one, where it is not a slot, and where that costs more than it saves,
+                    // the two stay apart.
                     DevBuf& o1 = t.bufs[items[i + 1].bufs[0].id];
                     bool clash = false;
                     for (void* q : ptrs) clash = clash || q == o1.ptr;
                     void* own = nullptr;
-                    if (clash && items[i + 1].bufs[0].slot >= 0) {
+                    if (clash && items[i + 1].bufs[0].slot >= 0 && gemm_joins_moved(dev, *plan)) {
                         if (dev->alloc(o1.bytes, &own) == ANL_OK) { t.owned.push_back(own); o1.ptr = own; clash = false; }
                         else cudaGetLastError();
                     }

@@ -228,6 +228,7 @@ bool gemm_fusable(const Plan& plan);
 bool gemm_pair_shape(const Plan& plan);
 // 0: the plan does not run on the one-CTA kernel; 1: it does, and adds all of K in one go; more: in slices or chunks
 int gemm_small_parts(const Plan& plan);
+bool gemm_joins_moved(anl_device* dev, const Plan& plan);
 bool gemm_tf32_eligible(const Plan& plan);
 int gemm_tf32_source(const Plan& plan, std::string& out, std::string& note);
 void gemm_shape(const Plan& plan, int64_t* M, int64_t* N, int64_t* K);

@@ -72,3 +72,28 @@ def test_replays_with_new_inputs(order, cols):
         assert np.isfinite(y).all() and np.abs(y).max() > 1e-3
         assert np.array_equal(y, want[k % len(feeds)])
     assert not np.array_equal(want[0], want[1])
+
+
+# one wave of tile pairs and of whole 128 x 128 tiles: apart; more pairs than fit at once, narrower tiles: joined
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,width,moves", [(1536, 2304, 0), (2304, 2304, 1), (2048, 1024, 0), (1024, 1024, 1), (2048, 2048, 1)])
+def test_outputs_move_where_that_pays(rows, width, moves):
+    R.reset()
+    before, R.MATERIALIZE_CONTRACTION_OPERANDS = R.MATERIALIZE_CONTRACTION_OPERANDS, "auto"
+    try:
+        h = Tensor.new_leaf((rows, width), dtypes.float16).set_data(W.normal(74, 0, rows * width))
+        w = W.normal(74, 1, width * width) * np.float32(1.5 / np.sqrt(width))
+        for _ in range(3):
+            h = nn.gelu_tanh(h.matmul(Tensor.new_leaf((width, width), dtypes.float16).set_data(w).permute((1, 0))))
+        items, ids = R.build_schedule([h])
+    finally:
+        R.MATERIALIZE_CONTRACTION_OPERANDS = before
+    inputs, got = leaf_inputs([h]), []
+    for flags in (0, Device.NO_EPILOGUE_FUSION):
+        dev = Device(0, flags)
+        try:
+            got.append(dev.replay(items, inputs)[ids[0]].copy())
+            assert dev.stats()["epilogues_fused"] == (0 if flags else 2 + moves)
+        finally:
+            dev.close()
+    assert np.isfinite(got[0]).all() and np.abs(got[0]).max() > 0.1 and np.array_equal(*got)
