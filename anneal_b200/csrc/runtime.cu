@@ -757,6 +757,7 @@ static std::shared_ptr<FusedEpilogue> fused_epilogue_for(anl_device* dev, const 
     return fe;
 }
 
+constexpr size_t kMovedBytes = 128u << 20;       // of outputs that leave their slots in one schedule: about the L2
 int run_items(anl_device* dev, const std::vector<Item>& items, const Bindings& binds, Table& t, cudaStream_t stream, bool keep_scratch = false) {
     CodegenOpts opts; opts.debug_bounds = (dev->flags & ANL_OPEN_DEBUG_BOUNDS) != 0;
     // A parameter may only be updated once every kernel of this schedule that reads it has been
@@ -908,6 +909,7 @@ int run_items(anl_device* dev, const std::vector<Item>& items, const Bindings& b
         pending.reads = std::move(reads); pending.writes = std::move(writes); pending.after = std::move(after); pending.item = i;
         return may_wait(next, pending.writes) ? ANL_OK : flush();
     };
+    size_t moved_bytes = 0;                                // outputs that have left their slots
     for (size_t i = 0; i < items.size(); i++) {
         const Item& it = items[i];
         if (absorbed.count(i)) if (int rc = flush()) return rc;
@@ -972,13 +974,14 @@ int run_items(anl_device* dev, const std::vector<Item>& items, const Bindings& b
                     // contraction is over when its consumer starts, gives every second layer of a forward pass its input's
                     // slot.  Such an output moves to a block of its own (a launch of 2.7 us and a round trip of the
                     // activations saved, 32 x 4096 in f16); without one, where it is not a slot, and where that costs more than it saves,
-                    // the two stay apart.
+                    // the two stay apart.  The block is held to the end of the call, or as long as the graph, so what moves is
+                    // bounded: a deep forward pass holds its two slots and kMovedBytes, not half of its activations.
                     DevBuf& o1 = t.bufs[items[i + 1].bufs[0].id];
                     bool clash = false;
                     for (void* q : ptrs) clash = clash || q == o1.ptr;
                     void* own = nullptr;
-                    if (clash && items[i + 1].bufs[0].slot >= 0 && gemm_joins_moved(dev, *plan)) {
-                        if (dev->alloc(o1.bytes, &own) == ANL_OK) { t.owned.push_back(own); o1.ptr = own; clash = false; }
+                    if (clash && items[i + 1].bufs[0].slot >= 0 && moved_bytes + o1.bytes <= kMovedBytes && gemm_joins_moved(dev, *plan)) {
+                        if (dev->alloc(o1.bytes, &own) == ANL_OK) { t.owned.push_back(own); o1.ptr = own; clash = false; moved_bytes += o1.bytes; }
                         else cudaGetLastError();
                     }
                     if (clash) fe.reset();
