@@ -160,7 +160,6 @@ constexpr int BATCH = SPLITS > 1 || CHUNK ? 1 : 4;
 static_assert(!CFG_A_MN || CFG_PROWS == 128, "an m-contiguous operand is staged whole");
 static_assert(!CFG_B_MN || NT % 64 == 0, "an n-contiguous operand is staged in boxes of 64");
 
-
 __device__ __forceinline__ void umma_f16(unsigned tmem_d, unsigned long long adesc, unsigned long long bdesc, unsigned idesc, unsigned accumulate) {
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
@@ -427,89 +426,85 @@ __device__ __forceinline__ void run(const TensorMap& map_a, const TensorMap& map
 #if CFG_EPI
             if (j0 > 0 || CHUNK) load_operands(j0);
 #endif
+            float4 a[BATCH][SPLITS], b[BATCH][SPLITS];
+            int trow[BATCH], tcol[BATCH];
+            bool on[BATCH];
 #pragma unroll
-            {
-                constexpr int h = 0;
-                float4 a[BATCH][SPLITS], b[BATCH][SPLITS];
-                int trow[BATCH], tcol[BATCH];
-                bool on[BATCH];
+            for (int q = 0; q < BATCH; q++) {
+                on[q] = piece(j0 + q, trow[q], tcol[q]);
+                if (!on[q]) continue;
+                const float* const at = tile + trow[q] * LDT + tcol[q];
+                if (SPLITS == 1) { a[q][0] = *reinterpret_cast<const float4*>(at); b[q][0] = *reinterpret_cast<const float4*>(at + 4); }
+                else {
 #pragma unroll
-                for (int q = 0; q < BATCH; q++) {
-                    on[q] = piece(j0 + h + q, trow[q], tcol[q]);
-                    if (!on[q]) continue;
-                    const float* const at = tile + trow[q] * LDT + tcol[q];
-                    if (SPLITS == 1) { a[q][0] = *reinterpret_cast<const float4*>(at); b[q][0] = *reinterpret_cast<const float4*>(at + 4); }
-                    else {
-#pragma unroll
-                        for (int r = 0; r < SPLITS; r++) { const unsigned p = map_to_cta(smem_u32(at), r); a[q][r] = ld_cluster_f4(p); b[q][r] = ld_cluster_f4(p + 16); }
-                    }
+                    for (int r = 0; r < SPLITS; r++) { const unsigned p = map_to_cta(smem_u32(at), r); a[q][r] = ld_cluster_f4(p); b[q][r] = ld_cluster_f4(p + 16); }
                 }
+            }
 #pragma unroll
-                for (int q = 0; q < BATCH; q++) {
-                    const int j = j0 + h + q, row = m0 + trow[q], col = n0 + tcol[q];
+            for (int q = 0; q < BATCH; q++) {
+                const int j = j0 + q, row = m0 + trow[q], col = n0 + tcol[q];
 #if !CFG_TF32
-                    if ((j & 3) == 0) {
+                if ((j & 3) == 0) {
 #pragma unroll
-                        for (int e = 0; e < 8; e++) x[e] = 0.0f;
-                    }
+                    for (int e = 0; e < 8; e++) x[e] = 0.0f;
+                }
 #endif
-                    if (on[q]) {
-                        float s[8] = {a[q][0].x, a[q][0].y, a[q][0].z, a[q][0].w, b[q][0].x, b[q][0].y, b[q][0].z, b[q][0].w};
+                if (on[q]) {
+                    float s[8] = {a[q][0].x, a[q][0].y, a[q][0].z, a[q][0].w, b[q][0].x, b[q][0].y, b[q][0].z, b[q][0].w};
 #pragma unroll
-                        for (int r = 1; r < SPLITS; r++) { s[0] += a[q][r].x; s[1] += a[q][r].y; s[2] += a[q][r].z; s[3] += a[q][r].w; s[4] += b[q][r].x; s[5] += b[q][r].y; s[6] += b[q][r].z; s[7] += b[q][r].w; }
-                        const size_t off = (size_t)row * g.N + col;
+                    for (int r = 1; r < SPLITS; r++) { s[0] += a[q][r].x; s[1] += a[q][r].y; s[2] += a[q][r].z; s[3] += a[q][r].w; s[4] += b[q][r].x; s[5] += b[q][r].y; s[6] += b[q][r].z; s[7] += b[q][r].w; }
+                    const size_t off = (size_t)row * g.N + col;
 #if CFG_TF32
-                        float* const d = (float*)g.d_raw + off;
-                        if ((g.N & 3) == 0) {
-                            *reinterpret_cast<float4*>(d) = make_float4(s[0], s[1], s[2], s[3]);
-                            if (col + 4 < g.N) *reinterpret_cast<float4*>(d + 4) = make_float4(s[4], s[5], s[6], s[7]);
-                        } else {
+                    float* const d = (float*)g.d_raw + off;
+                    if ((g.N & 3) == 0) {
+                        *reinterpret_cast<float4*>(d) = make_float4(s[0], s[1], s[2], s[3]);
+                        if (col + 4 < g.N) *reinterpret_cast<float4*>(d + 4) = make_float4(s[4], s[5], s[6], s[7]);
+                    } else {
 #pragma unroll
-                            for (int e = 0; e < 8; e++) if (col + e < g.N) d[e] = s[e];
-                        }
-#else
-                        uint4 T;
-                        __half2* const t2 = reinterpret_cast<__half2*>(&T);
-#pragma unroll
-                        for (int e = 0; e < 4; e++) t2[e] = __floats2half2_rn(s[2 * e], s[2 * e + 1]);     // the single narrowing
-                        if (vec_ok) {
-                            if (d_raw) *reinterpret_cast<uint4*>(d_raw + off) = T;
-#if CFG_EPI
-                            uint4 O;
-                            epi8_(row, col, t2, reinterpret_cast<__half2*>(&O), g.ep, raw[h + q]);
-                            *reinterpret_cast<uint4*>(d_out + off) = O;
-                            T = O;
-#endif
-                            if (g.colsum) {
-#pragma unroll
-                                for (int e = 0; e < 4; e++) { const float2 f = __half22float2(t2[e]); x[2 * e] += f.x; x[2 * e + 1] += f.y; }
-                            }
-                        } else {
-                            // row stride not a multiple of 16 bytes (no fused consumer on this route)
-#pragma unroll
-                            for (int e = 0; e < 4; e++) {
-                                if (col + 2 * e < g.N) d_raw[off + 2 * e] = __low2half(t2[e]);
-                                if (col + 2 * e + 1 < g.N) d_raw[off + 2 * e + 1] = __high2half(t2[e]);
-                            }
-                        }
-#endif
+                        for (int e = 0; e < 8; e++) if (col + e < g.N) d[e] = s[e];
                     }
-#if !CFG_TF32
-                    if (g.colsum && (j & 3) == 3) {
-                        // the eight lanes of a column piece hold rows i * 8 + lane / 4: their sums, across the lanes
+#else
+                    uint4 T;
+                    __half2* const t2 = reinterpret_cast<__half2*>(&T);
 #pragma unroll
-                        for (int o = 4; o <= 16; o <<= 1)
+                    for (int e = 0; e < 4; e++) t2[e] = __floats2half2_rn(s[2 * e], s[2 * e + 1]);     // the single narrowing
+                    if (vec_ok) {
+                        if (d_raw) *reinterpret_cast<uint4*>(d_raw + off) = T;
+#if CFG_EPI
+                        uint4 O;
+                        epi8_(row, col, t2, reinterpret_cast<__half2*>(&O), g.ep, raw[q]);
+                        *reinterpret_cast<uint4*>(d_out + off) = O;
+                        T = O;
+#endif
+                        if (g.colsum) {
 #pragma unroll
-                            for (int e = 0; e < 8; e++) x[e] += __shfl_xor_sync(0xffffffffu, x[e], o);
-                        const int row0 = m0 + (trow[q] & ~31);
-                        if (lane < 4 && trow[q] < BM && row0 < g.M && col < g.N) {        // warps past the last unit have rows past the tile
-                            float* const cs = g.colsum + (size_t)(row0 >> 5) * g.N + col;
+                            for (int e = 0; e < 4; e++) { const float2 f = __half22float2(t2[e]); x[2 * e] += f.x; x[2 * e + 1] += f.y; }
+                        }
+                    } else {
+                        // row stride not a multiple of 16 bytes (no fused consumer on this route)
 #pragma unroll
-                            for (int e = 0; e < 8; e++) cs[e] = x[e];
+                        for (int e = 0; e < 4; e++) {
+                            if (col + 2 * e < g.N) d_raw[off + 2 * e] = __low2half(t2[e]);
+                            if (col + 2 * e + 1 < g.N) d_raw[off + 2 * e + 1] = __high2half(t2[e]);
                         }
                     }
 #endif
                 }
+#if !CFG_TF32
+                if (g.colsum && (j & 3) == 3) {
+                    // the eight lanes of a column piece hold rows i * 8 + lane / 4: their sums, across the lanes
+#pragma unroll
+                    for (int o = 4; o <= 16; o <<= 1)
+#pragma unroll
+                        for (int e = 0; e < 8; e++) x[e] += __shfl_xor_sync(0xffffffffu, x[e], o);
+                    const int row0 = m0 + (trow[q] & ~31);
+                    if (lane < 4 && trow[q] < BM && row0 < g.M && col < g.N) {        // warps past the last unit have rows past the tile
+                        float* const cs = g.colsum + (size_t)(row0 >> 5) * g.N + col;
+#pragma unroll
+                        for (int e = 0; e < 8; e++) cs[e] = x[e];
+                    }
+                }
+#endif
             }
         }
     }
