@@ -836,7 +836,8 @@ __global__ void __launch_bounds__(256) colsum_finish(const float* __restrict__ p
     // A warp owns 8 columns (a sector), its four groups of lanes a contiguous quarter of the parts each (ascending, eight loads in
     // flight), and the four sums are added in order.  No shared memory: beside a two-CTA contraction, which leaves
     // 1.5 KB of an SM's, these blocks find a place at once; with 1 KB of their own they ran before the next
-    // contraction instead of beside it (step of 8192 rows, 4 x 4096 wide, 2746 -> 2726 us).
+    // contraction instead of beside it (step of 8192 rows, 4 x 4096 wide, at burst clocks 2746 -> 2726 us; at those of a long run
+    // no more than two runs differ by).
     enter_kernel();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, group = lane >> 3;
     const int col = (blockIdx.x * 8 + warp) * 8 + (lane & 7);
